@@ -66,29 +66,35 @@ template <typename C>
 __device__ __forceinline__ C csub(C a, C b) {
     return cx<C>(a.x - b.x, a.y - b.y);
 }
-// FP32: one packed instruction adds or subtracts both parts (the same two
-// rounded operations, the same bits). The single-tile real transforms are
-// bound by instruction issue (order 12: 73 instructions per complex point,
-// issue slots 61-65% busy), so the halved add count shows there: RFFT<float>
-// order 12 x 8192 forward + squared magnitudes 123.8 -> 119.9 us, backward
-// 88.8 -> 83.3, the STFT of 131069 such frames 881 -> 829 us. (Complex
-// products stay scalar: packing them needs duplicated operands, whose moves
-// cost what the packing saves.)
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) {
-    float2 r;
-    asm("{\n .reg .b64 a, b, r;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n add.rn.f32x2 r, a, b;\n"
-        " mov.b64 {%0, %1}, r;\n}"
-        : "=f"(r.x), "=f"(r.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return r;
+// Sum and difference of a butterfly: with PK, FP32 values go through one
+// packed instruction (both halves rounded as the scalar ones round them: the
+// same bits). The packed form halves the issue slots but ties the values
+// to register pairs, so each kernel says which suits it (TileCfg::kPack).
+template <bool PK, typename C>
+__device__ __forceinline__ C badd(C a, C b) {
+    if constexpr (PK && sizeof(C) == 8) {
+        C r;
+        asm("{\n .reg .b64 a, b, r;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n add.rn.f32x2 r, a, b;\n"
+            " mov.b64 {%0, %1}, r;\n}"
+            : "=f"(r.x), "=f"(r.y)
+            : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+        return r;
+    } else {
+        return cadd(a, b);
+    }
 }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) {
-    float2 r;
-    asm("{\n .reg .b64 a, b, r;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n sub.rn.f32x2 r, a, b;\n"
-        " mov.b64 {%0, %1}, r;\n}"
-        : "=f"(r.x), "=f"(r.y)
-        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return r;
+template <bool PK, typename C>
+__device__ __forceinline__ C bsub(C a, C b) {
+    if constexpr (PK && sizeof(C) == 8) {
+        C r;
+        asm("{\n .reg .b64 a, b, r;\n mov.b64 a, {%2, %3};\n mov.b64 b, {%4, %5};\n sub.rn.f32x2 r, a, b;\n"
+            " mov.b64 {%0, %1}, r;\n}"
+            : "=f"(r.x), "=f"(r.y)
+            : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+        return r;
+    } else {
+        return csub(a, b);
+    }
 }
 // a - i*b
 template <typename C>
@@ -116,63 +122,63 @@ __device__ __forceinline__ C cswap(C a) {
 // Radix-4 butterfly of the first Stockham pass (no twiddles), in place:
 // a_q = x[j + q*N/4] in, a_m = DFT4 output m out
 // (src/common/zldsp_fft_common_radix.hpp:192-238).
-template <typename C>
+template <bool PK = true, typename C>
 __device__ __forceinline__ void bfly4_first(C& a0, C& a1, C& a2, C& a3) {
-    const C t0 = cadd(a0, a2), t1 = csub(a0, a2);
-    const C t2 = cadd(a1, a3), t3 = csub(a1, a3);
-    a0 = cadd(t0, t2);
+    const C t0 = badd<PK>(a0, a2), t1 = bsub<PK>(a0, a2);
+    const C t2 = badd<PK>(a1, a3), t3 = bsub<PK>(a1, a3);
+    a0 = badd<PK>(t0, t2);
     a1 = csub_i(t1, t3);
-    a2 = csub(t0, t2);
+    a2 = bsub<PK>(t0, t2);
     a3 = cadd_i(t1, t3);
 }
 
 // Twiddled radix-4 DIT butterfly, in place (src/common/zldsp_fft_common_radix.hpp:103-156).
-template <typename C>
+template <bool PK = true, typename C>
 __device__ __forceinline__ void bfly4_tw(C& a0, C& a1, C& a2, C& a3, C w1, C w2, C w3) {
     const C t1 = cmul_tw(a1, w1);
     const C t3 = cmul_tw(a3, w3);
-    const C s2 = cadd(t1, t3), s3 = csub(t1, t3);
+    const C s2 = badd<PK>(t1, t3), s3 = bsub<PK>(t1, t3);
     const C t2 = cmul_tw(a2, w2);
-    const C s0 = cadd(a0, t2), s1 = csub(a0, t2);
-    a0 = cadd(s0, s2);
+    const C s0 = badd<PK>(a0, t2), s1 = bsub<PK>(a0, t2);
+    a0 = badd<PK>(s0, s2);
     a1 = csub_i(s1, s3);
-    a2 = csub(s0, s2);
+    a2 = bsub<PK>(s0, s2);
     a3 = cadd_i(s1, s3);
 }
 
 // Radix-8 butterfly of the first Stockham pass, in place: a_q = x[j + q*N/8]
 // in, a_p = DFT8 output p out. The W8 factors use 1/sqrt(2) formed as the
 // double quotient rounded to F (src/common/zldsp_fft_common_radix.hpp:495-568).
-template <typename C>
+template <bool PK = true, typename C>
 __device__ __forceinline__ void bfly8_first(C* a) {
     using F = decltype(C::x);
     const F c = (F)(1.0 / 1.4142135623730951);
-    const C t0 = cadd(a[0], a[4]), t1 = csub(a[0], a[4]);
-    const C t2 = cadd(a[2], a[6]), t3 = csub(a[2], a[6]);
-    const C y00 = cadd(t0, t2), y02 = csub(t0, t2);
+    const C t0 = badd<PK>(a[0], a[4]), t1 = bsub<PK>(a[0], a[4]);
+    const C t2 = badd<PK>(a[2], a[6]), t3 = bsub<PK>(a[2], a[6]);
+    const C y00 = badd<PK>(t0, t2), y02 = bsub<PK>(t0, t2);
     const C y01 = csub_i(t1, t3), y03 = cadd_i(t1, t3);
-    const C u0 = cadd(a[1], a[5]), u1 = csub(a[1], a[5]);
-    const C u2 = cadd(a[3], a[7]), u3 = csub(a[3], a[7]);
-    const C y10 = cadd(u0, u2), y12 = csub(u0, u2);
+    const C u0 = badd<PK>(a[1], a[5]), u1 = bsub<PK>(a[1], a[5]);
+    const C u2 = badd<PK>(a[3], a[7]), u3 = bsub<PK>(a[3], a[7]);
+    const C y10 = badd<PK>(u0, u2), y12 = bsub<PK>(u0, u2);
     const C y11 = csub_i(u1, u3), y13 = cadd_i(u1, u3);
     const C v1 = cx<C>(mul_rn(y11.x + y11.y, c), mul_rn(y11.y - y11.x, c));
     const C v2 = cx<C>(y12.y, -y12.x);
     const C v3 = cx<C>(mul_rn(y13.y - y13.x, c), mul_rn(-(y13.x + y13.y), c));
-    a[0] = cadd(y00, y10);
-    a[1] = cadd(y01, v1);
-    a[2] = cadd(y02, v2);
-    a[3] = cadd(y03, v3);
-    a[4] = csub(y00, y10);
-    a[5] = csub(y01, v1);
-    a[6] = csub(y02, v2);
-    a[7] = csub(y03, v3);
+    a[0] = badd<PK>(y00, y10);
+    a[1] = badd<PK>(y01, v1);
+    a[2] = badd<PK>(y02, v2);
+    a[3] = badd<PK>(y03, v3);
+    a[4] = bsub<PK>(y00, y10);
+    a[5] = bsub<PK>(y01, v1);
+    a[6] = bsub<PK>(y02, v2);
+    a[7] = bsub<PK>(y03, v3);
 }
 
-template <typename C>
+template <bool PK = true, typename C>
 __device__ __forceinline__ void bfly2(C& a0, C& a1) {
     const C t = a0;
-    a0 = cadd(t, a1);
-    a1 = csub(t, a1);
+    a0 = badd<PK>(t, a1);
+    a1 = bsub<PK>(t, a1);
 }
 
 // Twiddle W_N^t from the unified table T[t] = exp(-2*pi*i*t/N), t < 3N/4

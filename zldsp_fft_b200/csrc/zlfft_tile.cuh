@@ -168,6 +168,19 @@ struct TileCfg {
     // Register budget: enough resident CTAs for ~96 registers per thread in
     // FP32 (the last group's 15 complex twiddles stay in registers), ~128 in FP64.
     static constexpr int REGS = sizeof(F) == 4 ? (((OP == kC2CFwd || OP == kC2CBwd) && P >= 10) ? 128 : 96) : 128;
+    // Packed sums and differences (badd): where fewer issue slots outweigh the
+    // register pairs they need. Measured packed against scalar per order and
+    // operation, FP32, complex order P (transforms of 256 MiB, us): forward
+    // RFFT gains 1-9% from P = 8 up (P = 11: 112.2 -> 106.2, P = 14: 221.1 ->
+    // 204.3) except the squared magnitudes at P = 13 (149.5 -> 152.5); backward
+    // at P = 9, 11 and 12 (162.4 -> 155.8, 163.4 -> 153.3, 164.8 -> 155.2), not at
+    // 13 (214.6 -> 227.6); CFFT at P = 11 and 14 (210.8 -> 188.4, 362.8 -> 350.6),
+    // not at 12-13, whose fast form loses 6-10% (265.0 -> 293.0), nor below 11
+    // (memory bound; up to 3% slower).
+    static constexpr bool kPack =
+        sizeof(F) == 4 && ((OP == kR2CFwd && P >= 8) || (OP == kR2CSqrMag && P >= 8 && P != 13) ||
+                           (OP == kC2RBwd && (P == 9 || P == 11 || P == 12)) ||
+                           ((OP == kC2CFwd || OP == kC2CBwd) && (P == 11 || P == 14)));
     // Staging buffer for the next tile's input, filled by TMA bulk copies
     // while the current tile computes (not for the RFFT backward, whose
     // pre-step reads the bins).
@@ -320,30 +333,30 @@ __device__ __forceinline__ void group_load_tw(const C* tw, uint32_t k, C* w) {
 
 // Runs the stages of a group on the R registers r[] of one butterfly.
 // Output register s then holds output mu(s) (see group_mu).
-template <int R, int FIRST, typename C>
+template <int R, int FIRST, bool PK = true, typename C>
 __device__ __forceinline__ void group_compute(C* r, const C* w) {
     if constexpr (R == 2) {
-        bfly2(r[0], r[1]);
+        bfly2<PK>(r[0], r[1]);
     } else if constexpr (R == 8) {
-        bfly8_first(r);
+        bfly8_first<PK>(r);
     } else if constexpr (R == 4) {
         if constexpr (FIRST) {
-            bfly4_first(r[0], r[1], r[2], r[3]);
+            bfly4_first<PK>(r[0], r[1], r[2], r[3]);
         } else {
-            bfly4_tw(r[0], r[1], r[2], r[3], w[0], w[1], w[2]);
+            bfly4_tw<PK>(r[0], r[1], r[2], r[3], w[0], w[1], w[2]);
         }
     } else {  // R == 16: two radix-4 stages
         constexpr int o = FIRST ? 0 : 3;
         if constexpr (FIRST) {
 #pragma unroll
-            for (int a = 0; a < 4; ++a) bfly4_first(r[a], r[a + 4], r[a + 8], r[a + 12]);
+            for (int a = 0; a < 4; ++a) bfly4_first<PK>(r[a], r[a + 4], r[a + 8], r[a + 12]);
         } else {
 #pragma unroll
-            for (int a = 0; a < 4; ++a) bfly4_tw(r[a], r[a + 4], r[a + 8], r[a + 12], w[0], w[1], w[2]);
+            for (int a = 0; a < 4; ++a) bfly4_tw<PK>(r[a], r[a + 4], r[a + 8], r[a + 12], w[0], w[1], w[2]);
         }
 #pragma unroll
         for (int m = 0; m < 4; ++m)
-            bfly4_tw(r[4 * m], r[4 * m + 1], r[4 * m + 2], r[4 * m + 3], w[o + 3 * m], w[o + 3 * m + 1],
+            bfly4_tw<PK>(r[4 * m], r[4 * m + 1], r[4 * m + 2], r[4 * m + 3], w[o + 3 * m], w[o + 3 * m + 1],
                      w[o + 3 * m + 2]);
     }
 }
@@ -351,30 +364,30 @@ __device__ __forceinline__ void group_compute(C* r, const C* w) {
 // As group_compute, loading each butterfly's twiddles from the table right
 // before use (short live ranges; used where the twiddles are not held in
 // registers across transforms).
-template <int P, int R, int L, int FIRST, typename C>
+template <int P, int R, int L, int FIRST, bool PK = true, typename C>
 __device__ __forceinline__ void group_compute_ld(C* r, uint32_t k, const C* tws) {
     constexpr int L0 = stage_l0(P);
     if constexpr (R == 4 && !FIRST) {
         const C* t = tws + (L - L0) + k;
-        bfly4_tw(r[0], r[1], r[2], r[3], tw_load(t, 0), tw_load(t, L), tw_load(t, 2 * L));
+        bfly4_tw<PK>(r[0], r[1], r[2], r[3], tw_load(t, 0), tw_load(t, L), tw_load(t, 2 * L));
     } else if constexpr (R == 16) {
         if constexpr (FIRST) {
 #pragma unroll
-            for (int a = 0; a < 4; ++a) bfly4_first(r[a], r[a + 4], r[a + 8], r[a + 12]);
+            for (int a = 0; a < 4; ++a) bfly4_first<PK>(r[a], r[a + 4], r[a + 8], r[a + 12]);
         } else {
             const C* t = tws + (L - L0) + k;
             const C w1 = tw_load(t, 0), w2 = tw_load(t, L), w3 = tw_load(t, 2 * L);
 #pragma unroll
-            for (int a = 0; a < 4; ++a) bfly4_tw(r[a], r[a + 4], r[a + 8], r[a + 12], w1, w2, w3);
+            for (int a = 0; a < 4; ++a) bfly4_tw<PK>(r[a], r[a + 4], r[a + 8], r[a + 12], w1, w2, w3);
         }
         const C* t2 = tws + (4 * L - L0) + k;
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
-            bfly4_tw(r[4 * m], r[4 * m + 1], r[4 * m + 2], r[4 * m + 3], tw_load(t2, m * L),
+            bfly4_tw<PK>(r[4 * m], r[4 * m + 1], r[4 * m + 2], r[4 * m + 3], tw_load(t2, m * L),
                      tw_load(t2, m * L + 4 * L), tw_load(t2, m * L + 8 * L));
         }
     } else {
-        group_compute<R, FIRST>(r, (const C*)nullptr);
+        group_compute<R, FIRST, PK>(r, (const C*)nullptr);
     }
 }
 
@@ -439,7 +452,7 @@ __device__ __forceinline__ void group16_fast_tw(uint32_t k, const C* tws, C& w1,
     w4 = tw_load(tws, (uint32_t)L - L0 + k);
 }
 
-template <typename C>
+template <bool PK = true, typename C>
 __device__ __forceinline__ void group16_fast_w(C* r, const C w1, const C w4) {
     using F = decltype(C::x);
     const C w2 = cmul_tw(w1, w1), w3 = cmul_tw(w1, w2);
@@ -453,7 +466,7 @@ __device__ __forceinline__ void group16_fast_w(C* r, const C w1, const C w4) {
         r[rho] = cmul_tw(r[rho], w);
     }
 #pragma unroll
-    for (int a = 0; a < 4; ++a) bfly4_first(r[a], r[a + 4], r[a + 8], r[a + 12]);
+    for (int a = 0; a < 4; ++a) bfly4_first<PK>(r[a], r[a + 4], r[a + 8], r[a + 12]);
     // W_16^j = exp(-2 pi i j / 16) for j = a * m
     const C c1 = cx<C>((F)0.92387953251128674, (F)-0.38268343236508978);
     const C c2 = cx<C>((F)0.70710678118654752, (F)-0.70710678118654752);
@@ -461,17 +474,17 @@ __device__ __forceinline__ void group16_fast_w(C* r, const C w1, const C w4) {
     const C c4 = cx<C>((F)0, (F)-1);
     const C c6 = cx<C>((F)-0.70710678118654752, (F)-0.70710678118654752);
     const C c9 = cx<C>((F)-0.92387953251128674, (F)0.38268343236508978);
-    bfly4_first(r[0], r[1], r[2], r[3]);
-    bfly4_tw(r[4], r[5], r[6], r[7], c1, c2, c3);
-    bfly4_tw(r[8], r[9], r[10], r[11], c2, c4, c6);
-    bfly4_tw(r[12], r[13], r[14], r[15], c3, c6, c9);
+    bfly4_first<PK>(r[0], r[1], r[2], r[3]);
+    bfly4_tw<PK>(r[4], r[5], r[6], r[7], c1, c2, c3);
+    bfly4_tw<PK>(r[8], r[9], r[10], r[11], c2, c4, c6);
+    bfly4_tw<PK>(r[12], r[13], r[14], r[15], c3, c6, c9);
 }
 
-template <int P, int L, typename C>
+template <int P, int L, bool PK = true, typename C>
 __device__ __forceinline__ void group16_fast(C* r, uint32_t k, const C* tws) {
     C w1, w4;
     group16_fast_tw<P, L>(k, tws, w1, w4);
-    group16_fast_w(r, w1, w4);
+    group16_fast_w<PK>(r, w1, w4);
 }
 
 // ---------------------------------------------------------------- the tile worker
@@ -489,6 +502,8 @@ template <typename F, int P, int OP, int IL, int OL, int BLOCK = 128, bool GATHE
 struct TileWorker {
     using Cfg = TileCfg<F, P, OP, BLOCK, EM>;
     using C = Cx<F>;
+    // (the fast form of order 11 is 2% slower packed: 173.7 -> 177.1 us)
+    static constexpr bool kPack = Cfg::kPack && !(FAST && P == 11 && (OP == kC2CFwd || OP == kC2CBwd));
     static constexpr int N = Cfg::N, E = Cfg::E, T = Cfg::T, TPC = Cfg::TPC, NG = Cfg::NG;
     static constexpr bool kFwd = (OP == kC2CFwd || OP == kR2CFwd || OP == kR2CSqrMag);
     static constexpr bool kR2C = (OP == kR2CFwd || OP == kR2CSqrMag);
@@ -803,17 +818,17 @@ struct TileWorker {
                         }
                         // ---- compute
                         if constexpr (kLast && kLastReg) {
-                            group_compute<G.R, G.first>(v, wl);
+                            group_compute<G.R, G.first, kPack>(v, wl);
                         } else {
 #pragma unroll
                             for (int u = 0; u < NB; ++u) {
                                 const int b = (kLast ? b_last : lt) + u * T;
                                 if constexpr (fast_group<G, kLast>()) {  // fast-twiddle form, hoisted twiddles
-                                    group16_fast_w(v + u * G.R, fw[GI][0], fw[GI][1]);
+                                    group16_fast_w<kPack>(v + u * G.R, fw[GI][0], fw[GI][1]);
                                 } else if constexpr (FAST && G.R == 16 && !G.first) {
-                                    group16_fast<P, G.L>(v + u * G.R, (uint32_t)(b % G.L), tws);
+                                    group16_fast<P, G.L, kPack>(v + u * G.R, (uint32_t)(b % G.L), tws);
                                 } else {
-                                    group_compute_ld<P, G.R, G.L, G.first>(v + u * G.R, (uint32_t)(b % G.L), tws);
+                                    group_compute_ld<P, G.R, G.L, G.first, kPack>(v + u * G.R, (uint32_t)(b % G.L), tws);
                                 }
                             }
                         }
