@@ -283,6 +283,17 @@ __device__ __forceinline__ void discard_l2_line(const void* p) {
     asm volatile("discard.global.L2 [%0], 128;" ::"l"(p) : "memory");
 }
 
+// ---------------------------------------------------------------- dependent launches
+// Launches on one stream may overlap: a kernel launched with launch_dependent
+// (zlfft_launch.cuh) starts once every CTA of the one before it has called
+// pdl_trigger (or ended), sets up its barriers and twiddle registers, and
+// waits in pdl_wait until the kernel before it has completed and its writes
+// are visible. Every thread calls pdl_wait before it touches the caller's
+// buffers or scratch; only the plan's own tables, written before the plan
+// was handed out, may be read ahead of it. Both are no-ops in a plain launch.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Device error word bits (read back by the host with zlfft_plan_device_status).
 constexpr int kDevErrWaitTimeout = 1;
 

@@ -93,6 +93,8 @@ __global__ void __launch_bounds__(IstftCfg<F, P>::T, IstftCfg<F, P>::MINB)
     const long long m1 = (m0 + o.run < o.blocks) ? m0 + o.run : o.blocks;
     const C zero = cx<C>((F)0, (F)0);
     for (int i = (int)threadIdx.x; i < N; i += T) ring[i] = zero;
+    pdl_wait();
+    pdl_trigger();
     __syncthreads();
     const long long f0 = (m0 - o.k + 1 > 0) ? m0 - o.k + 1 : 0;
     const long long f1 = (m1 - 1 < o.n_frames - 1) ? m1 - 1 : o.n_frames - 1;
@@ -132,9 +134,8 @@ cudaError_t launch_istft(const TileArgs& a, const IstftArgs& o, cudaStream_t str
     if (run < 1) run = 1;
     oo.run = run;
     const long long grid = (o.blocks + run - 1) / run;
-    kern<<<(unsigned)grid, Cfg::T, Cfg::SMEM, stream>>>(a, oo);
     if (ctx.launches) ++*ctx.launches;
-    return cudaGetLastError();
+    return launch_dependent(kern, (unsigned)grid, Cfg::T, Cfg::SMEM, stream, a, oo);
 }
 
 // [complex order][input layout]; null where the order has no ISTFT kernel

@@ -34,6 +34,25 @@ struct LaunchCtx {
     std::atomic<size_t>* launches;  // incremented per kernel launch
 };
 
+// A launch that may begin while the kernel before it on the stream ends (see
+// pdl_wait): its launch latency, barrier set-up and twiddle loads overlap that
+// kernel's last tiles.
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*kern)(P...), unsigned grid, int threads, size_t smem, cudaStream_t stream,
+                             const A&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 using TileLaunchFn = cudaError_t (*)(const TileArgs&, cudaStream_t, const LaunchCtx&);
 
 struct TileTable {
@@ -57,9 +76,8 @@ cudaError_t launch_tile(const TileArgs& a, cudaStream_t stream, const LaunchCtx&
     const long long tiles = (a.batch + Cfg::TPC - 1) / Cfg::TPC;
     const long long cap = (long long)ctx.num_sms * blocks_per_sm;
     const unsigned grid = (unsigned)(tiles < cap ? tiles : cap);
-    kern<<<grid, Cfg::THREADS, Cfg::SMEM, stream>>>(a);
     if (ctx.launches) ++*ctx.launches;
-    return cudaGetLastError();
+    return launch_dependent(kern, grid, Cfg::THREADS, Cfg::SMEM, stream, a);
 }
 
 // ------------------------------------------------------------------ gathered tile launches

@@ -1016,8 +1016,12 @@ __global__ void __launch_bounds__(TileCfg<F, P, OP>::THREADS, TileCfg<F, P, OP>:
                 fence_mbar_init();
             }
             __syncthreads();
-            issue(blockIdx.x);
         }
+    }
+    pdl_trigger();  // the next kernel may set up in the slots this one's CTAs leave
+    pdl_wait();     // the caller's buffers may be the kernel before us's until here
+    if constexpr (Cfg::kTMA || Cfg::kTMA1) {
+        if (use_tma) issue(blockIdx.x);
     }
     uint32_t phase = 0;
     // backward RFFT: bins staged by cp.async, one tile ahead
