@@ -547,14 +547,15 @@ cudaError_t launch_split(const zlfft_plan_s* p, int dop, int out_layout, const v
     const dim3 grid = pair_grid(p, M, batch);
     const C* zc = static_cast<const C*>(z);
     const C* rw = static_cast<const C*>(p->d_rw);
+    cudaError_t e;
     if (dop == zlfft::kR2CSqrMag)
-        zlfft::rfft_split_kernel<F, zlfft::kR2CSqrMag, zlfft::kAoS><<<grid, 256, 0, st>>>(zc, o0, o1, rw, M, batch, M, out_stride, go0, go1);
+        e = zlfft::launch_dependent(zlfft::rfft_split_kernel<F, zlfft::kR2CSqrMag, zlfft::kAoS>, grid, 256, 0, st, zc, o0, o1, rw, M, batch, M, out_stride, go0, go1);
     else if (out_layout == ZLFFT_AOS)
-        zlfft::rfft_split_kernel<F, zlfft::kR2CFwd, zlfft::kAoS><<<grid, 256, 0, st>>>(zc, o0, o1, rw, M, batch, M, out_stride, go0, go1);
+        e = zlfft::launch_dependent(zlfft::rfft_split_kernel<F, zlfft::kR2CFwd, zlfft::kAoS>, grid, 256, 0, st, zc, o0, o1, rw, M, batch, M, out_stride, go0, go1);
     else
-        zlfft::rfft_split_kernel<F, zlfft::kR2CFwd, zlfft::kSoA><<<grid, 256, 0, st>>>(zc, o0, o1, rw, M, batch, M, out_stride, go0, go1);
+        e = zlfft::launch_dependent(zlfft::rfft_split_kernel<F, zlfft::kR2CFwd, zlfft::kSoA>, grid, 256, 0, st, zc, o0, o1, rw, M, batch, M, out_stride, go0, go1);
     if (ctx.launches) ++*ctx.launches;
-    return cudaGetLastError();
+    return e;
 }
 
 template <typename F>
@@ -565,12 +566,13 @@ cudaError_t launch_pre(const zlfft_plan_s* p, int in_layout, const void* i0, con
     const int M = 1 << p->cfft_order;
     const dim3 grid = pair_grid(p, M, batch);
     const C* rw = static_cast<const C*>(p->d_rw);
+    cudaError_t e;
     if (in_layout == ZLFFT_AOS)
-        zlfft::rfft_pre_kernel<F, zlfft::kAoS><<<grid, 256, 0, st>>>(i0, i1, static_cast<C*>(z), rw, M, batch, in_stride, M, gi0, gi1);
+        e = zlfft::launch_dependent(zlfft::rfft_pre_kernel<F, zlfft::kAoS>, grid, 256, 0, st, i0, i1, static_cast<C*>(z), rw, M, batch, in_stride, M, gi0, gi1);
     else
-        zlfft::rfft_pre_kernel<F, zlfft::kSoA><<<grid, 256, 0, st>>>(i0, i1, static_cast<C*>(z), rw, M, batch, in_stride, M, gi0, gi1);
+        e = zlfft::launch_dependent(zlfft::rfft_pre_kernel<F, zlfft::kSoA>, grid, 256, 0, st, i0, i1, static_cast<C*>(z), rw, M, batch, in_stride, M, gi0, gi1);
     if (ctx.launches) ++*ctx.launches;
-    return cudaGetLastError();
+    return e;
 }
 
 // Intermediates between passes are dropped from L2 once read (pass_kernel,

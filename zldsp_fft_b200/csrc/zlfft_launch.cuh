@@ -38,10 +38,10 @@ struct LaunchCtx {
 // pdl_wait): its launch latency, barrier set-up and twiddle loads overlap that
 // kernel's last tiles.
 template <typename... P, typename... A>
-cudaError_t launch_dependent(void (*kern)(P...), unsigned grid, int threads, size_t smem, cudaStream_t stream,
+cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t stream,
                              const A&... args) {
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
@@ -50,7 +50,7 @@ cudaError_t launch_dependent(void (*kern)(P...), unsigned grid, int threads, siz
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, args...);
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
 using TileLaunchFn = cudaError_t (*)(const TileArgs&, cudaStream_t, const LaunchCtx&);
@@ -281,9 +281,8 @@ cudaError_t launch_pass(const PassArgs& a_in, cudaStream_t stream, const LaunchC
     const long long items = a.batch * Cfg::CPT;
     const long long cap = (long long)ctx.num_sms * blocks_per_sm;
     const unsigned grid = (unsigned)(items < cap ? items : cap);
-    kern<<<grid, Cfg::THREADS, kSmem, stream>>>(a, maps);
     if (ctx.launches) ++*ctx.launches;
-    return cudaGetLastError();
+    return launch_dependent(kern, grid, Cfg::THREADS, kSmem, stream, a, maps);
 }
 
 template <typename F, int P, int PI, int S = 0>

@@ -345,9 +345,11 @@ __global__ void __launch_bounds__(PassCfg<F, P, PI, S>::THREADS, PassCfg<F, P, P
                 fence_mbar_init();
             }
             __syncthreads();
-            issue(blockIdx.x);
         }
     }
+    pdl_trigger();
+    pdl_wait();
+    if constexpr (Cfg::kTMA) issue(blockIdx.x);
     uint32_t phase = 0;
 
     // Fast form: the two table twiddles of each radix-16 group (a thread runs
@@ -715,8 +717,10 @@ __global__ void rfft_split_kernel(const Cx<F>* z, void* out0, void* out1, const 
                                   long long z_stride, long long out_stride, void* const* gout0, void* const* gout1) {
     using C = Cx<F>;
     const int k = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (k > M / 2) return;
+    if (k > M / 2) return;  // (a thread that has ended counts as having triggered and waited)
     const C w = k > 0 ? rw[k] : cx<C>((F)0, (F)0);  // the pair's twiddles, for every transform
+    pdl_trigger();
+    pdl_wait();
     for (long long tr = blockIdx.y; tr < batch; tr += gridDim.y) {
         const C* zt = z + tr * z_stride;
         constexpr int OL2 = (OP == kR2CSqrMag) ? (int)kAoS : LAYOUT;
@@ -754,8 +758,10 @@ __global__ void rfft_pre_kernel(const void* in0, const void* in1, Cx<F>* z, cons
                                 const void* const* gin1) {
     using C = Cx<F>;
     const int k = (int)(blockIdx.x * blockDim.x + threadIdx.x);
-    if (k > M / 2) return;
+    if (k > M / 2) return;  // (a thread that has ended counts as having triggered and waited)
     const C w = k > 0 ? rw[k] : cx<C>((F)0, (F)0);  // the pair's twiddles, for every transform
+    pdl_trigger();
+    pdl_wait();
     for (long long tr = blockIdx.y; tr < batch; tr += gridDim.y) {
         const CxIn<F, LAYOUT> in(gin0 ? gin0[tr] : in0, gin0 ? (gin1 ? gin1[tr] : nullptr) : in1,
                                  gin0 ? 0 : tr * in_stride);
