@@ -66,18 +66,34 @@ struct TileTable {
     TileLaunchFn fast[kTileTableP + 1][5][2];
 };
 
+// Transforms per thread. Two share their twiddle, window and split-twiddle
+// loads, their index arithmetic and their barriers (half of each per
+// transform), and give the scheduler two independent chains; they cost
+// registers (4 CTAs of 128 threads per SM instead of 5, with twice the
+// transforms in flight) and the separate staging buffer. Measured, complex
+// orders 9-11 (us, one -> two): STFT squared magnitudes 195.9 -> 182.1, 203.2 ->
+// 186.1, 208.2 -> 183.6; batched squared magnitudes at 10 and 11 102.0 -> 97.2,
+// 102.4 -> 97.6. The forward bins gain nothing (bound by their stores), and
+// from order 12 on the CTAs grow too large (order 13 106.0 -> 112.5).
+template <typename F, int P, int OP, bool WIN, bool FAST>
+constexpr int tile_nq() {
+    return sizeof(F) == 4 && P <= 11 && ((WIN && P >= 9) || (OP == kR2CSqrMag && P >= 10)) ? 2 : 1;
+}
+
 template <typename F, int P, int OP, int IL, int OL, bool WIN = false, bool FAST = false>
 cudaError_t launch_tile(const TileArgs& a, cudaStream_t stream, const LaunchCtx& ctx) {
-    using Cfg = TileCfg<F, P, OP>;
-    auto kern = tile_kernel<F, P, OP, IL, OL, false, WIN, FAST>;
+    constexpr int NQ = tile_nq<F, P, OP, WIN, FAST>();
+    using Cfg = TileCfg<F, P, OP, 128, 0, NQ>;
+    using Tabs = TileTabs<F, P, OP, WIN, FAST, Cfg>;
+    auto kern = tile_kernel<F, P, OP, IL, OL, false, WIN, FAST, NQ>;
     static ResidentSlots slots;
-    const int blocks_per_sm = resident_ctas(slots, [kern] { return occupancy_setup(kern, Cfg::THREADS, Cfg::SMEM); });
+    const int blocks_per_sm = resident_ctas(slots, [kern] { return occupancy_setup(kern, Cfg::THREADS, Tabs::SMEM); });
     if (a.batch <= 0) return cudaSuccess;
-    const long long tiles = (a.batch + Cfg::TPC - 1) / Cfg::TPC;
+    const long long tiles = (a.batch + Cfg::TPT - 1) / Cfg::TPT;
     const long long cap = (long long)ctx.num_sms * blocks_per_sm;
     const unsigned grid = (unsigned)(tiles < cap ? tiles : cap);
     if (ctx.launches) ++*ctx.launches;
-    return launch_dependent(kern, grid, Cfg::THREADS, Cfg::SMEM, stream, a);
+    return launch_dependent(kern, grid, Cfg::THREADS, Tabs::SMEM, stream, a);
 }
 
 // ------------------------------------------------------------------ gathered tile launches
@@ -91,14 +107,15 @@ struct GatherTable {
 template <typename F, int P, int OP, bool FAST = false>
 cudaError_t launch_tile_gather(const TileArgs& a, cudaStream_t stream, const LaunchCtx& ctx) {
     using Cfg = TileCfg<F, P, OP>;
+    using Tabs = TileTabs<F, P, OP, false, FAST, Cfg>;
     auto kern = tile_kernel<F, P, OP, kAoS, kAoS, true, false, FAST>;
     static ResidentSlots slots;
-    const int blocks_per_sm = resident_ctas(slots, [kern] { return occupancy_setup(kern, Cfg::THREADS, Cfg::SMEM); });
+    const int blocks_per_sm = resident_ctas(slots, [kern] { return occupancy_setup(kern, Cfg::THREADS, Tabs::SMEM); });
     if (a.batch <= 0) return cudaSuccess;
-    const long long tiles = (a.batch + Cfg::TPC - 1) / Cfg::TPC;
+    const long long tiles = (a.batch + Cfg::TPT - 1) / Cfg::TPT;
     const long long cap = (long long)ctx.num_sms * blocks_per_sm;
     const unsigned grid = (unsigned)(tiles < cap ? tiles : cap);
-    kern<<<grid, Cfg::THREADS, Cfg::SMEM, stream>>>(a);
+    kern<<<grid, Cfg::THREADS, Tabs::SMEM, stream>>>(a);
     if (ctx.launches) ++*ctx.launches;
     return cudaGetLastError();
 }

@@ -107,6 +107,13 @@ __host__ __device__ constexpr int ilog2c(long long x) {
     return r;
 }
 
+// Per-stage twiddle tables: the radix-4 stage with sub-length L (twiddles
+// W_{4L}^{qk}, q = 1..3, k < L) occupies 3L consecutive entries at offset
+// L - L0, q-major, where L0 is the first twiddled stage's sub-length (4 for
+// even orders, 8 for odd). Threads with consecutive k read consecutive
+// entries. The values are copies of the unified table's entries.
+__host__ __device__ constexpr int stage_l0(int P) { return (P % 2) ? 8 : 4; }
+
 struct TileArgs {
     const void* in0;
     const void* in1;
@@ -152,7 +159,7 @@ __device__ __forceinline__ C cmul_rn(const C x, const C h) {
     return cx<C>(sub_rn(mul_rn(x.x, h.x), mul_rn(x.y, h.y)), add_rn(mul_rn(x.x, h.y), mul_rn(x.y, h.x)));
 }
 
-template <typename F, int P, int OP = kC2CFwd, int BLOCK = 128, int EM = 0>
+template <typename F, int P, int OP = kC2CFwd, int BLOCK = 128, int EM = 0, int NQ = 1>
 struct TileCfg {
     using C = Cx<F>;
     static constexpr int N = 1 << P;
@@ -164,10 +171,11 @@ struct TileCfg {
     static constexpr int T = N / E;  // threads per transform
     static constexpr int TPC = T >= BLOCK ? 1 : BLOCK / T;
     static constexpr int THREADS = T * TPC;
-    static constexpr size_t XBYTES = (size_t)TPC * N * sizeof(C);  // exchange buffer
+    static constexpr int TPT = TPC * NQ;  // transforms per tile
+    static constexpr size_t XBYTES = (size_t)TPT * N * sizeof(C);  // exchange buffer
     // Register budget: enough resident CTAs for ~96 registers per thread in
     // FP32 (the last group's 15 complex twiddles stay in registers), ~128 in FP64.
-    static constexpr int REGS = sizeof(F) == 4 ? (((OP == kC2CFwd || OP == kC2CBwd) && P >= 10) ? 128 : 96) : 128;
+    static constexpr int REGS = NQ > 1 ? 128 : sizeof(F) == 4 ? (((OP == kC2CFwd || OP == kC2CBwd) && P >= 10) ? 128 : 96) : 128;
     // Packed sums and differences (badd): where fewer issue slots outweigh the
     // register pairs they need. Measured packed against scalar per order and
     // operation, FP32, complex order P (transforms of 256 MiB, us): forward
@@ -184,7 +192,7 @@ struct TileCfg {
     // Staging buffer for the next tile's input, filled by TMA bulk copies
     // while the current tile computes (not for the RFFT backward, whose
     // pre-step reads the bins).
-    static constexpr bool kTMA = P >= 4 && OP != kC2RBwd && 2 * XBYTES <= 200 * 1024;
+    static constexpr bool kTMA = P >= 4 && NQ == 1 && OP != kC2RBwd && 2 * XBYTES <= 200 * 1024;
     // Backward RFFT: the next tile's bins (TPC frames of N + 1 complex; SoA:
     // a re row then an im row per frame) are copied into the staging buffer
     // by cp.async while the current tile computes (dense bin arrays put odd
@@ -193,7 +201,7 @@ struct TileCfg {
     // 12: 2214 -> 2986, 13: 1848 -> 2346; but 8: 4533 -> 3770 and 10: 3910 ->
     // 3482, where the extra copy and shared-memory read outweigh the hidden
     // latency. FP64 keeps direct loads (its buffers would cost resident CTAs).
-    static constexpr size_t BBYTES = ((size_t)TPC * (N + 1) * sizeof(C) + 15) / 16 * 16;
+    static constexpr size_t BBYTES = ((size_t)TPT * (N + 1) * sizeof(C) + 15) / 16 * 16;
     static constexpr bool kStageBins = OP == kC2RBwd && sizeof(F) == 4 && (P == 9 || (P >= 11 && P <= 13)) &&
                                        XBYTES + BBYTES <= 200 * 1024;
     // 128 KB tiles (FP32 order 14, FP64 order 13: no room for a second
@@ -206,11 +214,51 @@ struct TileCfg {
     static constexpr Grp GL_ = tile_group(P, NG_ > 0 ? NG_ - 1 : 0);
     static constexpr bool kShufSplit = (OP == kR2CFwd || OP == kR2CSqrMag) && NG_ >= 2 && GL_.R == E && !GL_.first &&
                                        GL_.R == 16 && T >= 2;
-    static constexpr bool kTMA1 = !kTMA && (P == 14 || (sizeof(F) == 8 && P == 13)) &&
+    static constexpr bool kTMA1 = !kTMA && (NQ > 1 || P == 14 || (sizeof(F) == 8 && P == 13)) &&
                                   (OP == kC2CFwd || OP == kC2CBwd || kShufSplit) && XBYTES + 16 <= 200 * 1024;
     static constexpr size_t SMEM = kTMA ? 2 * XBYTES + 16 : (kTMA1 ? XBYTES + 16 : XBYTES + (kStageBins ? BBYTES : 0));
+    // twiddles of the groups before the last: the per-stage tables below the last group's
+    static constexpr int TW_MID = NG_ >= 2 && !GL_.first && GL_.L > stage_l0(P) ? GL_.L - stage_l0(P) : 0;
     static constexpr int NG = tile_num_groups(P);
     static constexpr int MINB = (65536 / (THREADS * REGS)) > 0 ? (65536 / (THREADS * REGS)) : 1;
+};
+
+// Tables a CTA copies into shared memory when it starts, behind the Cfg::SMEM
+// bytes of its buffers, and reads from there for every tile:
+// - kTabMid: the twiddles of the groups before the last (TW_MID entries);
+// - kTabRw: the RFFT split twiddles (N / 2 + 1);
+// - kTabWin: the STFT window (N pairs).
+// Each is copied where it costs no resident CTA. Read from global memory,
+// those loads missed behind the streaming data or at least waited for the L1
+// tag stage; measured (256 MiB of transforms, us, global -> shared): CFFT<float>
+// orders 10 / 12 / 13 190.6 -> 170.0, 238.3 -> 206.3, 294.3 -> 269.4, CFFT<double>
+// 12 161.2 -> 142.0; RFFT<float> order 13 forward 119.5 -> 104.7, squared
+// magnitudes 109.5 -> 99.0, backward 152.8 -> 129.1, order 10 backward 154.9 ->
+// 125.3. Not copied, because measured slower: anything below order 9 (memory
+// bound), the fast form's twiddles (two per group, in registers from order 12:
+// 198.8 -> 205.5; order 13, whose lone radix-4 group reads three, 267.4 -> 257.3),
+// those of the forward RFFT of complex order 13 (161.2 ->
+// 165.5), the 64 KB of split twiddles of complex order 14 (203.2 -> 219.9).
+enum TileTab : int { kTabMid = 1, kTabRw = 2, kTabWin = 4 };
+template <typename F, int P, int OP, bool WIN, bool FAST, class Cfg, size_t BASE = Cfg::SMEM, bool RWS = true>
+struct TileTabs {
+    static constexpr size_t CX = sizeof(Cx<F>);
+    static constexpr int N = 1 << P;
+    static constexpr size_t kSm = 227 * 1024;
+    static constexpr int CTAS = (int)(kSm / (BASE + 1024)) < Cfg::MINB ? (int)(kSm / (BASE + 1024)) : Cfg::MINB;
+    static constexpr size_t LIMIT = kSm / (CTAS > 0 ? CTAS : 1) - 1024;
+    static constexpr size_t mid_bytes = (size_t)Cfg::TW_MID * CX, rw_bytes = (size_t)(N / 2 + 1) * CX, win_bytes = N * CX;
+    static constexpr bool kReal = OP == kR2CFwd || OP == kR2CSqrMag || OP == kC2RBwd;
+    static constexpr bool kMid = Cfg::TW_MID > 0 && P >= 9 && (!FAST || P == 13) && !(OP == kR2CFwd && P == 13) &&
+                                 BASE + mid_bytes <= LIMIT;
+    static constexpr size_t OFF_MID = BASE;
+    static constexpr size_t OFF_RW = OFF_MID + (kMid ? mid_bytes : 0);
+    static constexpr bool kRw = RWS && kReal && P >= 9 && P <= 13 && OFF_RW + rw_bytes <= LIMIT;
+    static constexpr size_t OFF_WIN = OFF_RW + (kRw ? (rw_bytes + 15) / 16 * 16 : 0);
+    static constexpr bool kWin = WIN && P >= 9 && OFF_WIN + win_bytes <= LIMIT;
+    static constexpr size_t SMEM = OFF_WIN + (kWin ? win_bytes : 0);
+    static constexpr int TABS = (kMid ? kTabMid : 0) | (kRw ? kTabRw : 0) | (kWin ? kTabWin : 0);
+    static_assert(BASE % 16 == 0, "16-byte aligned table copies");
 };
 
 // XOR swizzle of a shared-memory slot index: keeps each 128-byte row, permutes
@@ -239,13 +287,6 @@ __device__ __forceinline__ uint32_t swz_mirror(uint32_t p) {
         return p ^ (((r / LW) & (16u / LW - 1u)) * LW);
     }
 }
-
-// Per-stage twiddle tables: the radix-4 stage with sub-length L (twiddles
-// W_{4L}^{qk}, q = 1..3, k < L) occupies 3L consecutive entries at offset
-// L - L0, q-major, where L0 is the first twiddled stage's sub-length (4 for
-// even orders, 8 for odd). Threads with consecutive k read consecutive
-// entries. The values are copies of the unified table's entries.
-__host__ __device__ constexpr int stage_l0(int P) { return (P % 2) ? 8 : 4; }
 
 // ---------------------------------------------------------------- global I/O
 // A complex stream seen from one transform's base: AoS is one array of
@@ -498,9 +539,10 @@ __device__ __forceinline__ void group16_fast(C* r, uint32_t k, const C* tws) {
 // swizzle (keep_idx), for a caller that stores the TPC transforms of a tile
 // together (the transposed store of the macro path, zlfft_macro.cuh).
 template <typename F, int P, int OP, int IL, int OL, int BLOCK = 128, bool GATHER = false, bool WIN = false,
-          bool FAST = false, bool KEEP = false, int EM = 0>
+          bool FAST = false, bool KEEP = false, int EM = 0, int NQ = 1, int TABS = 0>
 struct TileWorker {
-    using Cfg = TileCfg<F, P, OP, BLOCK, EM>;
+    using Cfg = TileCfg<F, P, OP, BLOCK, EM, NQ>;
+    static_assert(NQ == 1 || (!GATHER && !KEEP && OP != kC2RBwd), "several transforms per thread: contiguous, not C2R");
     using C = Cx<F>;
     // (the fast form of order 11 is 2% slower packed: 173.7 -> 177.1 us)
     static constexpr bool kPack = Cfg::kPack && !(FAST && P == 11 && (OP == kC2CFwd || OP == kC2CBwd));
@@ -530,8 +572,15 @@ struct TileWorker {
     // +8-10% at orders 12-13; at order 11 the longer live ranges cost 3-5%.)
     static constexpr bool kHoistFast = FAST && P >= 12;
     C fw[NG > 0 ? NG : 1][2];
+    // Tables read from copies in shared memory (TABS, bits of TileTab):
+    // kTabMid, kTabRw and kTabWin; null otherwise.
+    const C* t_mid;
+    const C* t_rw;
+    const C* t_win;
 
-    __device__ __forceinline__ TileWorker(const TileArgs& a, unsigned char* smem_raw) {
+    __device__ __forceinline__ TileWorker(const TileArgs& a, unsigned char* smem_raw, const C* mid = nullptr,
+                                          const C* rwt = nullptr, const C* wint = nullptr)
+        : t_mid(mid), t_rw(rwt), t_win(wint) {
         sm = reinterpret_cast<C*>(smem_raw);
         lt = (int)threadIdx.x % T;
         slot = (int)threadIdx.x / T;
@@ -613,10 +662,14 @@ struct TileWorker {
                                         const Sink& sink = Sink{}) {
         static_assert(!Sink::kActive || OP == kC2RBwd, "output sinks take backward RFFT samples");
         static_assert(!KEEP || (OP == kC2CFwd && (TPC & (TPC - 1)) == 0), "KEEP: forward C2C, power-of-two slots");
-        const C* stage = Cfg::kTMA1 ? sm : sm + (size_t)TPC * N;
-        const long long tr = tile * TPC + slot;
-        const bool valid = tr < a.batch;
-        // this slot's transform: contiguous (base + stride) or gathered pointers
+        const C* stage = Cfg::kTMA1 ? sm : sm + (size_t)Cfg::TPT * N;
+        // this slot's transforms, TPC apart (NQ of them): contiguous (base + stride) or gathered pointers
+        constexpr int QN = TPC * N;  // their distance in shared memory
+        const long long tr = tile * Cfg::TPT + slot;
+        bool valid_q[NQ];
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) valid_q[q] = tr + q * TPC < a.batch;
+        const bool valid = valid_q[0];
         const void* ib0 = a.in0;
         const void* ib1 = a.in1;
         void* ob0 = a.out0;
@@ -631,7 +684,11 @@ struct TileWorker {
             ob1 = a.gout1 ? a.gout1[g] : nullptr;
             ibase = obase = 0;
         }
-        C v[E];
+        // base of transform q (an invalid one's is never read or written)
+        auto ibq = [&](int q) -> long long { return q == 0 ? ibase : (tr + q * TPC) * a.in_stride; };
+        auto obq = [&](int q) -> long long { return q == 0 ? obase : (tr + q * TPC) * a.out_stride; };
+        C vq[NQ][E];
+        C(&v)[E] = vq[0];
 
         // ------------------------------------------------ input
         // Backward RFFT pre-step (execute.hpp:399-451): Z[p] from the bins at p
@@ -644,7 +701,7 @@ struct TileWorker {
         // the staged orders gained 3-9% (RFFT<float> backward order 13: 3018 ->
         // 3301 GB/s, order 14: 2342 -> 2558).
         constexpr bool kDirectPre = OP == kC2RBwd && NG >= 2 && Cfg::kStageBins && !Sink::kActive;
-        [[maybe_unused]] const C* rw = static_cast<const C*>(a.rw);
+        [[maybe_unused]] const C* rw = (TABS & kTabRw) ? t_rw : static_cast<const C*>(a.rw);
         [[maybe_unused]] const C* hf = static_cast<const C*>(sink.h);
         [[maybe_unused]] const F* sb = reinterpret_cast<const F*>(stage) + (size_t)slot * 2 * (N + 1);
         [[maybe_unused]] const CxIn<F, IL> bins(ib0, ib1, ibase);
@@ -726,7 +783,7 @@ struct TileWorker {
             }
             if constexpr (kR2C && WIN) {
                 {
-                    const C w = static_cast<const C*>(a.win)[0];
+                    const C w = ((TABS & kTabWin) ? t_win : static_cast<const C*>(a.win))[0];
                     x = cx<C>(mul_rn(x.x, w.x), mul_rn(x.y, w.y));
                 }
             }
@@ -754,43 +811,52 @@ struct TileWorker {
                             }
                         } else if constexpr (GI == 0 && OP != kC2RBwd) {
                             if (use_tma) {
-                                const C* sc = stage + (size_t)slot * N;
-                                const F* sf = reinterpret_cast<const F*>(sc);
 #pragma unroll
-                                for (int u = 0; u < NB; ++u) {
-                                    const int b = (kLast ? b_last : lt) + u * T;
-#pragma unroll
-                                    for (int rho = 0; rho < G.R; ++rho) {
-                                        const int pos = b + rho * (N / G.R);
-                                        C x = kSoAIn ? cx<C>(sf[pos], sf[N + pos]) : sc[pos];
-                                        v[u * G.R + rho] = kFwd ? x : cswap(x);
-                                    }
-                                }
-                                if constexpr (!Cfg::kTMA1) refill();
-                            } else {
-                                constexpr int IL2 = kR2C ? (int)kAoS : IL;
-                                const CxIn<F, IL2> in(ib0, ib1, ibase);
-#pragma unroll
-                                for (int u = 0; u < NB; ++u) {
-                                    const int b = (kLast ? b_last : lt) + u * T;
-#pragma unroll
-                                    for (int rho = 0; rho < G.R; ++rho) {
-                                        C x = valid ? in[b + rho * (N / G.R)] : cx<C>((F)0, (F)0);
-                                        v[u * G.R + rho] = kFwd ? x : cswap(x);
-                                    }
-                                }
-                            }
-                            if constexpr (kR2C && WIN) {  // STFT: window the frame as it is loaded
-                                {
-                                    const C* wp = static_cast<const C*>(a.win);
+                                for (int q = 0; q < NQ; ++q) {
+                                    const C* sc = stage + (size_t)slot * N + q * QN;
+                                    const F* sf = reinterpret_cast<const F*>(sc);
 #pragma unroll
                                     for (int u = 0; u < NB; ++u) {
                                         const int b = (kLast ? b_last : lt) + u * T;
 #pragma unroll
                                         for (int rho = 0; rho < G.R; ++rho) {
-                                            const C w = __ldg(wp + b + rho * (N / G.R));
-                                            C& x = v[u * G.R + rho];
-                                            x = cx<C>(mul_rn(x.x, w.x), mul_rn(x.y, w.y));
+                                            const int pos = b + rho * (N / G.R);
+                                            C x = kSoAIn ? cx<C>(sf[pos], sf[N + pos]) : sc[pos];
+                                            vq[q][u * G.R + rho] = kFwd ? x : cswap(x);
+                                        }
+                                    }
+                                }
+                                if constexpr (!Cfg::kTMA1) refill();
+                            } else {
+                                constexpr int IL2 = kR2C ? (int)kAoS : IL;
+#pragma unroll
+                                for (int q = 0; q < NQ; ++q) {
+                                    const CxIn<F, IL2> in(ib0, ib1, ibq(q));
+#pragma unroll
+                                    for (int u = 0; u < NB; ++u) {
+                                        const int b = (kLast ? b_last : lt) + u * T;
+#pragma unroll
+                                        for (int rho = 0; rho < G.R; ++rho) {
+                                            C x = valid_q[q] ? in[b + rho * (N / G.R)] : cx<C>((F)0, (F)0);
+                                            vq[q][u * G.R + rho] = kFwd ? x : cswap(x);
+                                        }
+                                    }
+                                }
+                            }
+                            if constexpr (kR2C && WIN) {  // STFT: window the frame as it is loaded
+                                {
+                                    const C* wp = (TABS & kTabWin) ? t_win : static_cast<const C*>(a.win);
+#pragma unroll
+                                    for (int u = 0; u < NB; ++u) {
+                                        const int b = (kLast ? b_last : lt) + u * T;
+#pragma unroll
+                                        for (int rho = 0; rho < G.R; ++rho) {
+                                            const C w = wp[b + rho * (N / G.R)];
+#pragma unroll
+                                            for (int q = 0; q < NQ; ++q) {
+                                                C& x = vq[q][u * G.R + rho];
+                                                x = cx<C>(mul_rn(x.x, w.x), mul_rn(x.y, w.y));
+                                            }
                                         }
                                     }
                                 }
@@ -808,8 +874,11 @@ struct TileWorker {
                                     } else {
                                         ix = sidx(pos);
                                     }
-                                    const C x = sm[ix];
-                                    v[u * G.R + rho] = (GI == 0 && OP == kC2RBwd) ? cswap(x) : x;
+#pragma unroll
+                                    for (int q = 0; q < NQ; ++q) {
+                                        const C x = sm[ix + q * QN];
+                                        vq[q][u * G.R + rho] = (GI == 0 && OP == kC2RBwd) ? cswap(x) : x;
+                                    }
                                 }
                             }
                             if constexpr (kLast && Cfg::kTMA1) {
@@ -817,18 +886,23 @@ struct TileWorker {
                             }
                         }
                         // ---- compute
-                        if constexpr (kLast && kLastReg) {
-                            group_compute<G.R, G.first, kPack>(v, wl);
-                        } else {
 #pragma unroll
-                            for (int u = 0; u < NB; ++u) {
-                                const int b = (kLast ? b_last : lt) + u * T;
-                                if constexpr (fast_group<G, kLast>()) {  // fast-twiddle form, hoisted twiddles
-                                    group16_fast_w<kPack>(v + u * G.R, fw[GI][0], fw[GI][1]);
-                                } else if constexpr (FAST && G.R == 16 && !G.first) {
-                                    group16_fast<P, G.L, kPack>(v + u * G.R, (uint32_t)(b % G.L), tws);
-                                } else {
-                                    group_compute_ld<P, G.R, G.L, G.first, kPack>(v + u * G.R, (uint32_t)(b % G.L), tws);
+                        for (int q = 0; q < NQ; ++q) {
+                            C* vv = vq[q];
+                            if constexpr (kLast && kLastReg) {
+                                group_compute<G.R, G.first, kPack>(vv, wl);
+                            } else {
+#pragma unroll
+                                for (int u = 0; u < NB; ++u) {
+                                    const int b = (kLast ? b_last : lt) + u * T;
+                                    if constexpr (fast_group<G, kLast>()) {  // fast-twiddle form, hoisted twiddles
+                                        group16_fast_w<kPack>(vv + u * G.R, fw[GI][0], fw[GI][1]);
+                                    } else if constexpr (FAST && G.R == 16 && !G.first) {
+                                        group16_fast<P, G.L, kPack>(vv + u * G.R, (uint32_t)(b % G.L), (TABS & kTabMid) && !kLast ? t_mid : tws);
+                                    } else {
+                                        group_compute_ld<P, G.R, G.L, G.first, kPack>(vv + u * G.R, (uint32_t)(b % G.L),
+                                                                                      (TABS & kTabMid) && !kLast ? t_mid : tws);
+                                    }
                                 }
                             }
                         }
@@ -851,7 +925,8 @@ struct TileWorker {
                                     } else {
                                         ix = sidx(pos);
                                     }
-                                    sm[ix] = v[u * G.R + s];
+#pragma unroll
+                                    for (int q = 0; q < NQ; ++q) sm[ix + q * QN] = vq[q][u * G.R + s];
                                 }
                             }
                             __syncthreads();
@@ -860,47 +935,51 @@ struct TileWorker {
                             // (lt ^ H) holds Z[N - b - mu*L] at slot 15 - mu (for the lanes
                             // holding b = 0 and b = L/2 the partner is the lane itself).
                             constexpr int L = G.L;
-                            C z[16];
 #pragma unroll
-                            for (int s = 0; s < 16; ++s) z[group_mu(G, s)] = v[s];
-                            const C* rw = static_cast<const C*>(a.rw);
-                            [[maybe_unused]] F* osq = static_cast<F*>(ob0) + obase;
+                            for (int q = 0; q < NQ; ++q) {
+                                const bool valid = valid_q[q];
+                                const CxOut<F, OL2> out(ob0, ob1, obq(q));
+                                [[maybe_unused]] F* osq = static_cast<F*>(ob0) + obq(q);
+                                C z[16];
 #pragma unroll
-                            for (int m = 0; m < 8; ++m) {
-                                C p;
-                                p.x = __shfl_xor_sync(0xffffffffu, z[15 - m].x, H);
-                                p.y = __shfl_xor_sync(0xffffffffu, z[15 - m].y, H);
-                                C z2 = p;
-                                const int k = b_last + m * L;
-                                if (lt == 0) {  // b = 0: pairs (m, 16 - m); m = 0 is DC/Nyquist
-                                    z2 = z[(16 - m) & 15];
-                                } else if (lt == H) {  // b = L/2: pairs (m, 15 - m) in this lane
-                                    z2 = z[15 - m];
-                                }
-                                if (valid && !(lt == 0 && m == 0)) {
-                                    const C w = rw[k];
-                                    const SplitOut<F> o = rfft_split<F>(z[m], z2, w.x, w.y);
-                                    if constexpr (OP == kR2CFwd) {
-                                        if (k != N / 2) out.put(k, cx<C>(o.xr_k, o.xi_k));
-                                        out.put(N - k, cx<C>(o.xr_m, o.xi_m));
-                                    } else {
-                                        if (k != N / 2) __stcs(osq + k, fma_rn(o.xr_k, o.xr_k, mul_rn(o.xi_k, o.xi_k)));
-                                        __stcs(osq + N - k, fma_rn(o.xr_m, o.xr_m, mul_rn(o.xi_m, o.xi_m)));
+                                for (int s = 0; s < 16; ++s) z[group_mu(G, s)] = vq[q][s];
+#pragma unroll
+                                for (int m = 0; m < 8; ++m) {
+                                    C p;
+                                    p.x = __shfl_xor_sync(0xffffffffu, z[15 - m].x, H);
+                                    p.y = __shfl_xor_sync(0xffffffffu, z[15 - m].y, H);
+                                    C z2 = p;
+                                    const int k = b_last + m * L;
+                                    if (lt == 0) {  // b = 0: pairs (m, 16 - m); m = 0 is DC/Nyquist
+                                        z2 = z[(16 - m) & 15];
+                                    } else if (lt == H) {  // b = L/2: pairs (m, 15 - m) in this lane
+                                        z2 = z[15 - m];
+                                    }
+                                    const C w = rw[k];  // outside the branch: the loads of all m go out together
+                                    if (valid && !(lt == 0 && m == 0)) {
+                                        const SplitOut<F> o = rfft_split<F>(z[m], z2, w.x, w.y);
+                                        if constexpr (OP == kR2CFwd) {
+                                            if (k != N / 2) out.put(k, cx<C>(o.xr_k, o.xi_k));
+                                            out.put(N - k, cx<C>(o.xr_m, o.xi_m));
+                                        } else {
+                                            if (k != N / 2) __stcs(osq + k, fma_rn(o.xr_k, o.xr_k, mul_rn(o.xi_k, o.xi_k)));
+                                            __stcs(osq + N - k, fma_rn(o.xr_m, o.xr_m, mul_rn(o.xi_m, o.xi_m)));
+                                        }
                                     }
                                 }
-                            }
-                            if (valid && lt == 0) {  // b = 0 also owns k = N/2 (slot 8) and DC/Nyquist
-                                const C w = rw[N / 2];
-                                const SplitOut<F> o = rfft_split<F>(z[8], z[8], w.x, w.y);
-                                const F dc = z[0].x + z[0].y, ny = z[0].x - z[0].y;
-                                if constexpr (OP == kR2CFwd) {
-                                    out.put(N / 2, cx<C>(o.xr_m, o.xi_m));
-                                    out.put(0, cx<C>(dc, (F)0));
-                                    out.put(N, cx<C>(ny, (F)0));
-                                } else {
-                                    __stcs(osq + N / 2, fma_rn(o.xr_m, o.xr_m, mul_rn(o.xi_m, o.xi_m)));
-                                    __stcs(osq, mul_rn(dc, dc));
-                                    __stcs(osq + N, mul_rn(ny, ny));
+                                if (valid && lt == 0) {  // b = 0 also owns k = N/2 (slot 8) and DC/Nyquist
+                                    const C w = rw[N / 2];
+                                    const SplitOut<F> o = rfft_split<F>(z[8], z[8], w.x, w.y);
+                                    const F dc = z[0].x + z[0].y, ny = z[0].x - z[0].y;
+                                    if constexpr (OP == kR2CFwd) {
+                                        out.put(N / 2, cx<C>(o.xr_m, o.xi_m));
+                                        out.put(0, cx<C>(dc, (F)0));
+                                        out.put(N, cx<C>(ny, (F)0));
+                                    } else {
+                                        __stcs(osq + N / 2, fma_rn(o.xr_m, o.xr_m, mul_rn(o.xi_m, o.xi_m)));
+                                        __stcs(osq, mul_rn(dc, dc));
+                                        __stcs(osq + N, mul_rn(ny, ny));
+                                    }
                                 }
                             }
                         } else if constexpr (KEEP) {
@@ -913,18 +992,24 @@ struct TileWorker {
                             }
                         } else {
 #pragma unroll
-                            for (int u = 0; u < NB; ++u) {
-                                const int b = b_last + u * T;  // J == 0 in the last group
+                            for (int q = 0; q < NQ; ++q) {
+                                const CxOut<F, OL2> outq(ob0, ob1, obq(q));
 #pragma unroll
-                                for (int s = 0; s < G.R; ++s) {
-                                    const int pos = b + group_mu(G, s) * G.L;
-                                    if constexpr (kR2C) {
-                                        sm[sidx(pos)] = v[u * G.R + s];
-                                    } else if (valid) {
-                                        if constexpr (Sink::kActive) {
-                                            sink.add(pos, cswap(v[u * G.R + s]));
-                                        } else {
-                                            out.put(pos, kFwd ? v[u * G.R + s] : cswap(v[u * G.R + s]));
+                                for (int u = 0; u < NB; ++u) {
+                                    const int b = b_last + u * T;  // J == 0 in the last group
+#pragma unroll
+                                    for (int s = 0; s < G.R; ++s) {
+                                        const int pos = b + group_mu(G, s) * G.L;
+                                        const C x = vq[q][u * G.R + s];
+                                        if constexpr (kR2C) {
+                                            static_assert(NQ == 1, "several transforms per thread: the shuffle split");
+                                            sm[sidx(pos)] = x;
+                                        } else if (valid_q[q]) {
+                                            if constexpr (Sink::kActive) {
+                                                sink.add(pos, cswap(x));
+                                            } else {
+                                                outq.put(pos, kFwd ? x : cswap(x));
+                                            }
                                         }
                                     }
                                 }
@@ -940,7 +1025,6 @@ struct TileWorker {
         if constexpr (kR2C && !kShufPost) {
             __syncthreads();
             if (valid) {
-                const C* rw = static_cast<const C*>(a.rw);
                 [[maybe_unused]] F* osq = static_cast<F*>(ob0) + obase;
                 for (int k = 1 + lt; k <= N / 2; k += T) {
                     const C w = rw[k];
@@ -973,37 +1057,50 @@ struct TileWorker {
 };
 
 // ---------------------------------------------------------------- the kernel
-template <typename F, int P, int OP, int IL, int OL, bool GATHER = false, bool WIN = false, bool FAST = false>
-__global__ void __launch_bounds__(TileCfg<F, P, OP>::THREADS, TileCfg<F, P, OP>::MINB) tile_kernel(const TileArgs a) {
-    using W = TileWorker<F, P, OP, IL, OL, 128, GATHER, WIN, FAST>;
-    using Cfg = typename W::Cfg;
+template <typename C>
+__device__ __forceinline__ void copy_table(C* dst, const C* src, int n) {
+    for (int i = (int)threadIdx.x; i < n; i += (int)blockDim.x) dst[i] = src[i];
+}
+
+template <typename F, int P, int OP, int IL, int OL, bool GATHER = false, bool WIN = false, bool FAST = false,
+          int NQ = 1>
+__global__ void __launch_bounds__(TileCfg<F, P, OP, 128, 0, NQ>::THREADS, TileCfg<F, P, OP, 128, 0, NQ>::MINB)
+    tile_kernel(const TileArgs a) {
+    using Cfg = TileCfg<F, P, OP, 128, 0, NQ>;
+    using Tabs = TileTabs<F, P, OP, WIN, FAST, Cfg>;
+    using W = TileWorker<F, P, OP, IL, OL, 128, GATHER, WIN, FAST, false, 0, NQ, Tabs::TABS>;
     using C = Cx<F>;
-    constexpr int N = Cfg::N, TPC = Cfg::TPC;
+    constexpr int N = Cfg::N, TPT = Cfg::TPT;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    W w(a, smem_raw);
+    C* t_mid = reinterpret_cast<C*>(smem_raw + Tabs::OFF_MID);
+    C* t_rw = reinterpret_cast<C*>(smem_raw + Tabs::OFF_RW);
+    C* t_win = reinterpret_cast<C*>(smem_raw + Tabs::OFF_WIN);
+    if constexpr (Tabs::kMid) copy_table(t_mid, static_cast<const C*>(a.tws), Cfg::TW_MID);
+    if constexpr (Tabs::kRw) copy_table(t_rw, static_cast<const C*>(a.rw), N / 2 + 1);
+    W w(a, smem_raw, t_mid, t_rw, t_win);
 
     // ---- TMA staging of each tile's input (one tile ahead)
     constexpr bool kSoAIn = W::kSoAIn;
-    C* stage = reinterpret_cast<C*>(smem_raw) + (Cfg::kTMA1 ? 0 : (size_t)TPC * N);
+    C* stage = reinterpret_cast<C*>(smem_raw) + (Cfg::kTMA1 ? 0 : (size_t)TPT * N);
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem_raw + Cfg::XBYTES * (Cfg::kTMA1 ? 1 : 2));
     // gathered transforms (AoS): one bulk copy from each transform's own pointer,
     // where the batch found every input 16-byte aligned (a.tma)
     const bool use_tma = (Cfg::kTMA || Cfg::kTMA1) && (!GATHER || !kSoAIn) && a.tma;
     auto issue = [&](long long t) {  // warp 0 issues the copies of tile t
-        if (!use_tma || threadIdx.x >= 32 || t * TPC >= a.batch) return;
-        const long long left = a.batch - t * TPC;
-        const int nvalid = (int)(left < TPC ? left : TPC);
+        if (!use_tma || threadIdx.x >= 32 || t * TPT >= a.batch) return;
+        const long long left = a.batch - t * TPT;
+        const int nvalid = (int)(left < TPT ? left : TPT);
         constexpr uint32_t kSlot = (uint32_t)(N * sizeof(C));
         if (threadIdx.x == 0) mbar_arrive_expect_tx(bar, kSlot * (uint32_t)nvalid);
         __syncwarp();
         for (int q = (int)threadIdx.x; q < nvalid; q += 32) {
-            const long long base = (t * TPC + q) * a.in_stride;
+            const long long base = (t * TPT + q) * a.in_stride;
             if constexpr (kSoAIn) {
                 F* dst = reinterpret_cast<F*>(stage + (size_t)q * N);
                 bulk_g2s(dst, static_cast<const F*>(a.in0) + base, kSlot / 2, bar);
                 bulk_g2s(dst + N, static_cast<const F*>(a.in1) + base, kSlot / 2, bar);
             } else if constexpr (GATHER) {
-                bulk_g2s(stage + (size_t)q * N, static_cast<const C*>(a.gin0[t * TPC + q]), kSlot, bar);
+                bulk_g2s(stage + (size_t)q * N, static_cast<const C*>(a.gin0[t * TPT + q]), kSlot, bar);
             } else {
                 bulk_g2s(stage + (size_t)q * N, static_cast<const C*>(a.in0) + base, kSlot, bar);
             }
@@ -1015,11 +1112,12 @@ __global__ void __launch_bounds__(TileCfg<F, P, OP>::THREADS, TileCfg<F, P, OP>:
                 mbar_init(bar, 1);
                 fence_mbar_init();
             }
-            __syncthreads();
         }
     }
     pdl_trigger();  // the next kernel may set up in the slots this one's CTAs leave
     pdl_wait();     // the caller's buffers may be the kernel before us's until here
+    if constexpr (Tabs::kWin) copy_table(t_win, static_cast<const C*>(a.win), N);
+    __syncthreads();  // barrier initialised, table copies complete
     if constexpr (Cfg::kTMA || Cfg::kTMA1) {
         if (use_tma) issue(blockIdx.x);
     }
@@ -1028,7 +1126,7 @@ __global__ void __launch_bounds__(TileCfg<F, P, OP>::THREADS, TileCfg<F, P, OP>:
     const bool use_stage = Cfg::kStageBins && !GATHER && a.tma;
     if (use_stage) w.stage_bins(a, blockIdx.x);
 
-    for (long long tile = blockIdx.x; tile * TPC < a.batch; tile += gridDim.x) {
+    for (long long tile = blockIdx.x; tile * TPT < a.batch; tile += gridDim.x) {
         if constexpr (Cfg::kTMA || Cfg::kTMA1) {
             if (use_tma) {
                 const bool ok = mbar_wait(bar, phase);
