@@ -234,11 +234,13 @@ struct TileCfg {
 // orders 10 / 12 / 13 190.6 -> 170.0, 238.3 -> 206.3, 294.3 -> 269.4, CFFT<double>
 // 12 161.2 -> 142.0; RFFT<float> order 13 forward 119.5 -> 104.7, squared
 // magnitudes 109.5 -> 99.0, backward 152.8 -> 129.1, order 10 backward 154.9 ->
-// 125.3. Not copied, because measured slower: anything below order 9 (memory
-// bound), the fast form's twiddles (two per group, in registers from order 12:
-// 198.8 -> 205.5; order 13, whose lone radix-4 group reads three, 267.4 -> 257.3),
-// those of the forward RFFT of complex order 13 (161.2 ->
-// 165.5), the 64 KB of split twiddles of complex order 14 (203.2 -> 219.9).
+// 125.3; the fast form, which kept its two twiddles per group in registers
+// before, order 13 269.8 -> 251.0, CFFT<double> 12 244.3 -> 226.8, RFFT<double> 13
+// 165.7 -> 130.1. Not copied, because measured slower: anything below order 9
+// (memory bound), the twiddles of the forward RFFT of complex order 13 (161.2 ->
+// 165.5) and of the fast form at order 14 (316.3 -> 324.0) and RFFT<double> 12
+// (116.4 -> 124.3), the 64 KB of split twiddles of complex order 14 (203.2 ->
+// 219.9).
 enum TileTab : int { kTabMid = 1, kTabRw = 2, kTabWin = 4 };
 template <typename F, int P, int OP, bool WIN, bool FAST, class Cfg, size_t BASE = Cfg::SMEM, bool RWS = true>
 struct TileTabs {
@@ -249,8 +251,8 @@ struct TileTabs {
     static constexpr size_t LIMIT = kSm / (CTAS > 0 ? CTAS : 1) - 1024;
     static constexpr size_t mid_bytes = (size_t)Cfg::TW_MID * CX, rw_bytes = (size_t)(N / 2 + 1) * CX, win_bytes = N * CX;
     static constexpr bool kReal = OP == kR2CFwd || OP == kR2CSqrMag || OP == kC2RBwd;
-    static constexpr bool kMid = Cfg::TW_MID > 0 && P >= 9 && (!FAST || P == 13) && !(OP == kR2CFwd && P == 13) &&
-                                 BASE + mid_bytes <= LIMIT;
+    static constexpr bool kMid = Cfg::TW_MID > 0 && P >= 9 && !(OP == kR2CFwd && P == 13) && !(FAST && P == 14) &&
+                                 !(FAST && kReal && sizeof(F) == 8 && P == 11) && BASE + mid_bytes <= LIMIT;
     static constexpr size_t OFF_MID = BASE;
     static constexpr size_t OFF_RW = OFF_MID + (kMid ? mid_bytes : 0);
     static constexpr bool kRw = RWS && kReal && P >= 9 && P <= 13 && OFF_RW + rw_bytes <= LIMIT;
@@ -566,11 +568,10 @@ struct TileWorker {
     const C* tws;
     int b_last;
     C wl[kLastTw > 0 ? kLastTw : 1];
-    // fast form, complex orders 12 and up: the two table twiddles of each
-    // radix-16 group that reads its twiddles (one butterfly per thread in such
-    // a group, at a per-thread constant k), loaded once per CTA. (Measured:
-    // +8-10% at orders 12-13; at order 11 the longer live ranges cost 3-5%.)
-    static constexpr bool kHoistFast = FAST && P >= 12;
+    // fast form of the orders from 12 whose middle twiddles are not in shared
+    // memory: the two table twiddles of each radix-16 group (one butterfly per
+    // thread in such a group, at a per-thread constant k), loaded once per CTA
+    static constexpr bool kHoistFast = FAST && P >= 12 && !(TABS & kTabMid);
     C fw[NG > 0 ? NG : 1][2];
     // Tables read from copies in shared memory (TABS, bits of TileTab):
     // kTabMid, kTabRw and kTabWin; null otherwise.
