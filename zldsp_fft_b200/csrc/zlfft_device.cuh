@@ -275,6 +275,17 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
     return false;
 }
 
+// Starts bringing [p, p + bytes) into L2 (the 16-byte aligned part of it),
+// issued by one thread.
+__device__ __forceinline__ void prefetch_l2(const void* p, size_t bytes) {
+    const uintptr_t a = (reinterpret_cast<uintptr_t>(p) + 15) & ~(uintptr_t)15;
+    const uintptr_t e = (reinterpret_cast<uintptr_t>(p) + bytes) & ~(uintptr_t)15;
+    if (e > a)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(__cvta_generic_to_global(reinterpret_cast<void*>(a))),
+                     "r"((uint32_t)(e - a))
+                     : "memory");
+}
+
 // Drops one 128-byte line of global memory from L2 without writing it back
 // (its contents become undefined): for intermediates that no later kernel
 // reads, so that the dead data does not cost DRAM write bandwidth when L2

@@ -45,13 +45,16 @@ template <typename F>
 struct OlaSink {
     using C = Cx<F>;
     static constexpr bool kActive = true;
-    const void* h;   // spectral filter (read by the pre-step) or null
+    const C* h;      // spectral filter (read by the pre-step)
+    const C* w;      // synthesis window pairs
+    bool has_h, has_w;
     C* ring;         // shared memory, N_c pairs
-    const C* w;      // synthesis window pairs or null
     uint32_t base;   // (f * hop / 2) mod N_c
     uint32_t mask;   // N_c - 1
+    __device__ __forceinline__ bool filtered() const { return has_h; }
+    __device__ __forceinline__ C filter(int k) const { return h[k]; }
     __device__ __forceinline__ void add(int pos, C x) const {
-        if (w) {
+        if (has_w) {
             const C ww = w[pos];
             x = cx<C>(mul_rn(x.x, ww.x), mul_rn(x.y, ww.y));
         }
@@ -60,82 +63,143 @@ struct OlaSink {
     }
 };
 
+// One CTA per SM of GROUPS groups of T threads, each a worker of its own: an
+// exchange buffer, a ring and a run of blocks. What the groups share is the
+// tables in shared memory, one copy per SM: the transform's middle twiddles
+// and split twiddles, the filter and the window, as many as fit without
+// costing a group. (A CTA per group, reading all four from global memory:
+// 1420 us for 131069 frames of order 12 at hop N / 4 against 1365, 319 against
+// 289 for 4096 frames of order 14. A copy per CTA would not fit.) The bins are
+// read directly: staging them costs a group.
 template <typename F, int P>
 struct IstftCfg {
     using C = Cx<F>;
     static constexpr int N = 1 << P;                  // complex points (frame length / 2)
-    static constexpr int T = N / tile_elems(P);       // one transform per CTA
+    static constexpr int T = N / tile_elems(P);       // threads per transform
     using Tile = TileCfg<F, P, kC2RBwd, (T > 0 ? T : 1)>;
-    // exchange, then the ring. The bins are read directly: staging them costs
-    // a resident CTA here and measured no faster (the frame rate of the
-    // transform bounds this kernel).
-    static constexpr size_t RING = Tile::XBYTES;
-    static constexpr size_t SMEM = RING + (size_t)N * sizeof(C);
+    static constexpr size_t RING = Tile::XBYTES;                    // a group's ring, behind its exchange
+    static constexpr size_t GBYTES = RING + (size_t)N * sizeof(C);  // bytes of a group
     // whole warps, and the exchange and ring in shared memory
-    static constexpr bool kOK = T >= 32 && Tile::TPC == 1 && SMEM <= 200 * 1024;
-    static_assert(!kOK || Tile::THREADS == T, "one transform per CTA of T threads");
-    static constexpr int MINB = Tile::MINB;
+    static constexpr bool kOK = T >= 32 && Tile::TPC == 1 && GBYTES <= 200 * 1024;
+    static_assert(!kOK || Tile::THREADS == T, "one transform per group of T threads");
+    static constexpr size_t kSm = 226 * 1024;
+    static constexpr int REGS = sizeof(F) == 4 && P <= 11 ? 96 : 128;
+    static constexpr int by_regs = 65536 / (REGS * (T > 0 ? T : 1)), by_smem = (int)(kSm / GBYTES);
+    static constexpr int G0 = by_regs < by_smem ? by_regs : by_smem;
+    static constexpr int G1 = G0 > 1024 / (T > 0 ? T : 1) ? 1024 / (T > 0 ? T : 1) : G0;
+    static constexpr int GROUPS = T > 32 && G1 > 15 ? 15 : (G1 > 0 ? G1 : 1);
+    static constexpr int THREADS = T * GROUPS;
+    static constexpr size_t BASE = GBYTES * GROUPS;
+    static constexpr size_t cxs = sizeof(C);
+    static constexpr size_t mid_b = Tile::TW_MID * cxs, rw_b = ((N / 2 + 1) * cxs + 15) / 16 * 16,
+                            h_b = ((N + 1) * cxs + 15) / 16 * 16, w_b = N * cxs;
+    static constexpr bool kMid = BASE + mid_b <= kSm;
+    static constexpr size_t O_MID = BASE, O_RW = O_MID + (kMid ? mid_b : 0);
+    static constexpr bool kRw = O_RW + rw_b <= kSm;
+    static constexpr size_t O_H = O_RW + (kRw ? rw_b : 0);
+    static constexpr bool kH = O_H + h_b <= kSm;
+    static constexpr size_t O_W = O_H + (kH ? h_b : 0);
+    static constexpr bool kW = O_W + w_b <= kSm;
+    static constexpr size_t SMEM = O_W + (kW ? w_b : 0);
+    static constexpr int TABS = (kMid ? kTabMid : 0) | (kRw ? kTabRw : 0);
 };
 
 template <typename F, int P, int IL>
-__global__ void __launch_bounds__(IstftCfg<F, P>::T, IstftCfg<F, P>::MINB)
-    istft_kernel(const TileArgs a, const IstftArgs o) {
+__global__ void __launch_bounds__(IstftCfg<F, P>::THREADS, 1) istft_kernel(const TileArgs a, const IstftArgs o) {
     using Cfg = IstftCfg<F, P>;
     using C = Cx<F>;
-    using W = TileWorker<F, P, kC2RBwd, IL, kAoS, Cfg::T>;
+    using W = TileWorker<F, P, kC2RBwd, IL, kAoS, Cfg::T, false, false, false, false, 0, 1, Cfg::TABS, true>;
     constexpr int N = Cfg::N, T = Cfg::T;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    W wk(a, smem_raw);
-    C* ring = reinterpret_cast<C*>(smem_raw + Cfg::RING);
+    const int grp = (int)threadIdx.x / T, lt = (int)threadIdx.x % T;
+    C* t_mid = reinterpret_cast<C*>(smem_raw + Cfg::O_MID);
+    C* t_rw = reinterpret_cast<C*>(smem_raw + Cfg::O_RW);
+    C* t_h = reinterpret_cast<C*>(smem_raw + Cfg::O_H);
+    C* t_w = reinterpret_cast<C*>(smem_raw + Cfg::O_W);
+    if constexpr (Cfg::kMid) copy_table(t_mid, static_cast<const C*>(a.tws), Cfg::Tile::TW_MID);
+    if constexpr (Cfg::kRw) copy_table(t_rw, static_cast<const C*>(a.rw), N / 2 + 1);
+    W wk(a, smem_raw + (size_t)grp * Cfg::GBYTES, t_mid, t_rw);
+    C* ring = reinterpret_cast<C*>(smem_raw + (size_t)grp * Cfg::GBYTES + Cfg::RING);
     C* sig = static_cast<C*>(o.sig);
     const long long hp = o.hop / 2;  // hop in sample pairs
-    const long long m0 = (long long)blockIdx.x * o.run;
-    const long long m1 = (m0 + o.run < o.blocks) ? m0 + o.run : o.blocks;
     const C zero = cx<C>((F)0, (F)0);
-    for (int i = (int)threadIdx.x; i < N; i += T) ring[i] = zero;
-    pdl_wait();
+    for (int i = lt; i < N; i += T) ring[i] = zero;
     pdl_trigger();
-    __syncthreads();
+    pdl_wait();
+    const long long m0 = ((long long)grp * gridDim.x + blockIdx.x) * o.run;
+    const long long m1 = (m0 + o.run < o.blocks) ? m0 + o.run : o.blocks;
     const long long f0 = (m0 - o.k + 1 > 0) ? m0 - o.k + 1 : 0;
     const long long f1 = (m1 - 1 < o.n_frames - 1) ? m1 - 1 : o.n_frames - 1;
-    OlaSink<F> sink{o.filt, ring, static_cast<const C*>(o.win), 0u, (uint32_t)(N - 1)};
+    // The bins come from HBM with nothing else to do meanwhile: one thread asks
+    // L2 for the next frame's before this one is transformed (1639 -> 1365 us for
+    // 131069 frames of order 12 at hop N / 4; with it the shared tables are worth
+    // 4% there, without it nothing).
+    auto prefetch = [&](long long f) {
+        if (lt != 0 || f > f1 || m0 >= m1) return;
+        if constexpr (IL == kSoA) {
+            prefetch_l2(static_cast<const F*>(a.in0) + f * a.in_stride, (N + 1) * sizeof(F));
+            prefetch_l2(static_cast<const F*>(a.in1) + f * a.in_stride, (N + 1) * sizeof(F));
+        } else {
+            prefetch_l2(static_cast<const C*>(a.in0) + f * a.in_stride, (N + 1) * sizeof(C));
+        }
+    };
+    prefetch(f0);
+    if (Cfg::kH && o.filt) copy_table(t_h, static_cast<const C*>(o.filt), N + 1);
+    if (Cfg::kW && o.win) copy_table(t_w, static_cast<const C*>(o.win), N);
+    __syncthreads();
+    if (m0 >= m1) return;  // (the groups meet at no barrier from here on)
+    OlaSink<F> sink{Cfg::kH ? t_h : static_cast<const C*>(o.filt), Cfg::kW ? t_w : static_cast<const C*>(o.win),
+                    o.filt != nullptr, o.win != nullptr, ring, 0u, (uint32_t)(N - 1)};
     for (long long f = f0; f <= f1; ++f) {
+        prefetch(f + 1);
         sink.base = (uint32_t)((f * hp) & (N - 1));
         wk.run(a, f, false, [] {}, sink);  // ends with a barrier: the frame is in the ring
-        // block f is final: write it when this CTA owns it, clear its slots
-        for (long long i = threadIdx.x; i < hp; i += T) {
+        // block f is final: write it when this group owns it, clear its slots
+        for (long long i = lt; i < hp; i += T) {
             const uint32_t r = (uint32_t)((f * hp + i) & (N - 1));
             if (f >= m0) sig[f * hp + i] = ring[r];
             ring[r] = zero;
         }
-        __syncthreads();
+        wk.sync();
     }
     // blocks after the last frame are final once every frame is in
     for (long long m = (f1 + 1 > m0 ? f1 + 1 : m0); m < m1; ++m)
-        for (long long i = threadIdx.x; i < hp; i += T) sig[m * hp + i] = ring[(uint32_t)((m * hp + i) & (N - 1))];
+        for (long long i = lt; i < hp; i += T) sig[m * hp + i] = ring[(uint32_t)((m * hp + i) & (N - 1))];
 }
 
 using IstftLaunchFn = cudaError_t (*)(const TileArgs&, const IstftArgs&, cudaStream_t, const LaunchCtx&);
 
-// One CTA per run of blocks. A run spans ~one wave of resident CTAs over the
-// output, and at least 4 (K - 1) blocks, so that the K - 1 frames each CTA
-// transforms ahead of its run add at most a quarter to the work.
+// One group per run of blocks. A full load takes one wave of the resident
+// groups, at least 4 (K - 1) blocks each, so that the K - 1 frames a group
+// transforms ahead of its run add at most a quarter to the work. A smaller
+// one weighs those frames against idle SMs: a run of `run` blocks costs
+// run + K - 1 frames, and a frame takes about 3 units of time on an SM whose
+// other groups idle, 2 g with g groups at work. Run r is group r / grid of CTA
+// r % grid, so that few runs still spread over all SMs.
 template <typename F, int P, int IL>
 cudaError_t launch_istft(const TileArgs& a, const IstftArgs& o, cudaStream_t stream, const LaunchCtx& ctx) {
     using Cfg = IstftCfg<F, P>;
     auto kern = istft_kernel<F, P, IL>;
     static ResidentSlots slots;
-    const int blocks_per_sm = resident_ctas(slots, [kern] { return occupancy_setup(kern, Cfg::T, Cfg::SMEM); });
+    (void)resident_ctas(slots, [kern] { return occupancy_setup(kern, Cfg::THREADS, Cfg::SMEM); });
     if (o.n_frames <= 0 || o.blocks <= 0) return cudaSuccess;
     IstftArgs oo = o;
-    const long long cap = (long long)ctx.num_sms * blocks_per_sm;
-    long long run = (o.blocks + cap - 1) / cap;
-    if (run < 4LL * (o.k - 1)) run = 4LL * (o.k - 1);
-    if (run < 1) run = 1;
+    const long long cap = (long long)ctx.num_sms * Cfg::GROUPS;
+    const long long rmin = (o.blocks + cap - 1) / cap;
+    long long run = rmin, best = -1;
+    for (long long r = rmin; r <= 4LL * (o.k - 1); ++r) {
+        const long long g = ((o.blocks + r - 1) / r + ctx.num_sms - 1) / ctx.num_sms;
+        const long long cost = (r + o.k - 1) * (2 * g > 3 ? 2 * g : 3);
+        if (best < 0 || cost < best) {
+            best = cost;
+            run = r;
+        }
+    }
     oo.run = run;
-    const long long grid = (o.blocks + run - 1) / run;
+    const long long groups = (o.blocks + run - 1) / run;
+    const long long grid = groups < ctx.num_sms ? groups : ctx.num_sms;
     if (ctx.launches) ++*ctx.launches;
-    return launch_dependent(kern, (unsigned)grid, Cfg::T, Cfg::SMEM, stream, a, oo);
+    return launch_dependent(kern, (unsigned)grid, Cfg::THREADS, Cfg::SMEM, stream, a, oo);
 }
 
 // [complex order][input layout]; null where the order has no ISTFT kernel

@@ -292,7 +292,7 @@ cudaError_t launch_pass(const PassArgs& a_in, cudaStream_t stream, const LaunchC
         }
     }
     static ResidentSlots slots;
-    constexpr size_t kSmem = SPLIT != 0 ? Cfg::SMEM_SPLIT : Cfg::SMEM;
+    constexpr size_t kSmem = (SPLIT != 0 ? Cfg::SMEM_SPLIT : Cfg::SMEM) + (FAST ? 0 : Cfg::TWBYTES);
     const int blocks_per_sm = resident_ctas(slots, [kern] { return occupancy_setup(kern, Cfg::THREADS, kSmem); });
     if (a.batch <= 0) return cudaSuccess;
     const long long items = a.batch * Cfg::CPT;

@@ -123,9 +123,18 @@ struct PassCfg {
     // The next item's input (a box of UPC units x R positions) is prefetched
     // by one 3-D tensor copy per 256 positions while the current item computes.
     static constexpr int RB = R < 256 ? R : 256;  // positions per box
+    // First pass, plain form, from 256 points: its twiddles depend on no unit,
+    // so each CTA copies them (the per-stage tables below L_OUT) to shared
+    // memory, behind the buffers. Measured, CFFT<float> plain (256-512 MiB, us):
+    // order 16 737.0 -> 726.5, 17 781.0 -> 759.6, 18 911.1 -> 837.8, CFFT<double> 18
+    // 1023.0 -> 947.3; the fast form (two loads per group) and the shorter first
+    // passes lose 1-4%.
+    static constexpr int TW = FIRST && R >= 256 ? R - stage_l0(P) : 0;
     static constexpr bool kTMA = SOFF + SBYTES + 16 + 1024 <= 200 * 1024;
     // (+1024: the buffers start at the first 1024-byte boundary of the dynamic
     // shared memory, as the swizzled output boxes of the first pass require)
+    static constexpr size_t TWOFF = kTMA ? SOFF + SBYTES + 16 : (XBYTES + 15) / 16 * 16;
+    static constexpr size_t TWBYTES = (size_t)TW * sizeof(C);  // added to SMEM by the plain form
     static constexpr size_t SMEM = (kTMA ? SOFF + SBYTES + 16 : XBYTES) + 1024;
     // Last pass with the RFFT split fused: the item's HALF low units (one box)
     // and a window of WIN = HALF + 2 units that holds their HALF mirrors
@@ -148,7 +157,7 @@ struct PassCfg {
     // Resident CTAs per SM: as many as the shared memory allows, within a
     // budget of 80 registers per thread in FP32 and 96 in FP64 (a cap of ~100
     // made the FP64 plain form spill).
-    static constexpr int SMEM_CTAS = (227 * 1024) / (int)(SMEM + 1024);
+    static constexpr int SMEM_CTAS = (227 * 1024) / (int)(SMEM + TWBYTES + 1024);
     static constexpr int REG_CTAS = 65536 / (THREADS * (sizeof(F) == 4 ? 80 : 96));
     static constexpr int MINB_ = SMEM_CTAS < REG_CTAS ? SMEM_CTAS : REG_CTAS;
     static constexpr int MINB = MINB_ > 0 ? MINB_ : 1;
@@ -347,6 +356,14 @@ __global__ void __launch_bounds__(PassCfg<F, P, PI, S>::THREADS, PassCfg<F, P, P
             __syncthreads();
         }
     }
+    constexpr bool kTw = Cfg::TW > 0 && !FAST;
+    const C* twl = tws;
+    if constexpr (kTw) {
+        C* t = reinterpret_cast<C*>(smem + Cfg::TWOFF);
+        copy_table(t, tws, Cfg::TW);
+        twl = t;
+        __syncthreads();
+    }
     pdl_trigger();
     pdl_wait();
     if constexpr (Cfg::kTMA) issue(blockIdx.x);
@@ -366,7 +383,7 @@ __global__ void __launch_bounds__(PassCfg<F, P, PI, S>::THREADS, PassCfg<F, P, P
                             static_assert(G.R == E, "one radix-16 butterfly per thread");
                             constexpr int ELL = G.L / L_IN;
                             const uint32_t kk = (uint32_t)(ku + L_IN * (tb % ELL));
-                            group16_fast_tw<P, G.L>(kk, tws, fw[GI][0], fw[GI][1]);
+                            group16_fast_tw<P, G.L>(kk, twl, fw[GI][0], fw[GI][1]);
                         }
                     }(),
                     ...);
@@ -479,7 +496,7 @@ __global__ void __launch_bounds__(PassCfg<F, P, PI, S>::THREADS, PassCfg<F, P, P
                         if constexpr (FAST && G.R == 16 && !G.first) {
                             group16_fast_w<PK>(v + i * G.R, fw[GI][0], fw[GI][1]);
                         } else {
-                            group_compute_ld<P, G.R, G.L, G.first, PK>(v + i * G.R, kk, tws);
+                            group_compute_ld<P, G.R, G.L, G.first, PK>(v + i * G.R, kk, twl);
                         }
                     }
                     // ---- outputs

@@ -145,11 +145,10 @@ struct TileArgs {
 // Output sink of the backward RFFT's last group. NoSink: the transform's
 // samples go to the output array. A sink with kActive (the overlap-add of
 // zlfft_istft.cuh) receives them instead, as add(pos, x) with x = real samples
-// 2 pos and 2 pos + 1, and may carry a spectral filter h (N + 1 bins,
-// multiplied into the bins as the pre-step reads them; null: none).
+// 2 pos and 2 pos + 1, and may carry a spectral filter (filtered(), filter(k),
+// k <= N: multiplied into the bins as the pre-step reads them).
 struct NoSink {
     static constexpr bool kActive = false;
-    const void* h = nullptr;
 };
 
 // Complex product with each operation rounded on its own:
@@ -541,7 +540,7 @@ __device__ __forceinline__ void group16_fast(C* r, uint32_t k, const C* tws) {
 // swizzle (keep_idx), for a caller that stores the TPC transforms of a tile
 // together (the transposed store of the macro path, zlfft_macro.cuh).
 template <typename F, int P, int OP, int IL, int OL, int BLOCK = 128, bool GATHER = false, bool WIN = false,
-          bool FAST = false, bool KEEP = false, int EM = 0, int NQ = 1, int TABS = 0>
+          bool FAST = false, bool KEEP = false, int EM = 0, int NQ = 1, int TABS = 0, bool GRP = false>
 struct TileWorker {
     using Cfg = TileCfg<F, P, OP, BLOCK, EM, NQ>;
     static_assert(NQ == 1 || (!GATHER && !KEEP && OP != kC2RBwd), "several transforms per thread: contiguous, not C2R");
@@ -584,7 +583,7 @@ struct TileWorker {
         : t_mid(mid), t_rw(rwt), t_win(wint) {
         sm = reinterpret_cast<C*>(smem_raw);
         lt = (int)threadIdx.x % T;
-        slot = (int)threadIdx.x / T;
+        slot = GRP ? 0 : (int)threadIdx.x / T;
         sbase = (uint32_t)slot * N;
         tw = static_cast<const C*>(a.tw);
         tws = static_cast<const C*>(a.tws);
@@ -603,6 +602,19 @@ struct TileWorker {
                     }(),
                     ...);
             }(std::make_integer_sequence<int, NG>{});
+        }
+    }
+
+    // Barrier over the threads that share this worker's exchange buffer: the
+    // CTA, or with GRP one of several independent groups of T threads in it
+    // (named barriers 1, 2, ...; a group of a warp needs none).
+    __device__ __forceinline__ void sync() const {
+        if constexpr (!GRP) {
+            __syncthreads();
+        } else if constexpr (T <= 32) {
+            __syncwarp();
+        } else {
+            asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / T), "n"(T) : "memory");
         }
     }
 
@@ -703,7 +715,6 @@ struct TileWorker {
         // 3301 GB/s, order 14: 2342 -> 2558).
         constexpr bool kDirectPre = OP == kC2RBwd && NG >= 2 && Cfg::kStageBins && !Sink::kActive;
         [[maybe_unused]] const C* rw = (TABS & kTabRw) ? t_rw : static_cast<const C*>(a.rw);
-        [[maybe_unused]] const C* hf = static_cast<const C*>(sink.h);
         [[maybe_unused]] const F* sb = reinterpret_cast<const F*>(stage) + (size_t)slot * 2 * (N + 1);
         [[maybe_unused]] const CxIn<F, IL> bins(ib0, ib1, ibase);
         [[maybe_unused]] auto bin = [&](int k) -> C {  // bin k, times the filter's bin k
@@ -722,7 +733,7 @@ struct TileWorker {
                 x = bins[k];
             }
             if constexpr (Sink::kActive) {
-                if (hf) x = cmul_rn(x, hf[k]);
+                if (sink.filtered()) x = cmul_rn(x, sink.filter(k));
             }
             return x;
         };
@@ -745,7 +756,7 @@ struct TileWorker {
             if constexpr (Cfg::kStageBins) {
                 if (use_tma) {  // this tile's bins are in the staging buffer
                     cp_async_wait_all();
-                    __syncthreads();
+                    sync();
                 }
             }
             if constexpr (!kDirectPre) {
@@ -762,7 +773,7 @@ struct TileWorker {
                     }
                     if (lt == 0) sm[sidx(0)] = prez(0);
                 }
-                __syncthreads();
+                sync();
                 if constexpr (Cfg::kStageBins) {
                     if (use_tma) refill();  // the staged bins are read: the next tile's may come in
                 }
@@ -909,7 +920,7 @@ struct TileWorker {
                         }
                         // ---- outputs
                         if constexpr (!kLast) {
-                            __syncthreads();
+                            sync();
                             if constexpr (GI == 0 && kDirectPre && Cfg::kStageBins) {
                                 if (use_tma) refill();  // the staged bins are read: the next tile's may come in
                             }
@@ -930,7 +941,7 @@ struct TileWorker {
                                     for (int q = 0; q < NQ; ++q) sm[ix + q * QN] = vq[q][u * G.R + s];
                                 }
                             }
-                            __syncthreads();
+                            sync();
                         } else if constexpr (kShufPost) {
                             // RFFT split from registers: z[mu] = Z[b + mu*L]; the partner lane
                             // (lt ^ H) holds Z[N - b - mu*L] at slot 15 - mu (for the lanes
@@ -984,7 +995,7 @@ struct TileWorker {
                                 }
                             }
                         } else if constexpr (KEEP) {
-                            __syncthreads();  // every input of the last group is read: the buffer is free
+                            sync();  // every input of the last group is read: the buffer is free
 #pragma unroll
                             for (int u = 0; u < NB; ++u) {
                                 const int b = b_last + u * T;
@@ -1024,7 +1035,7 @@ struct TileWorker {
         // ------------------------------------------------ RFFT forward split through shared memory
         // (orders without a shuffle-friendly last group)
         if constexpr (kR2C && !kShufPost) {
-            __syncthreads();
+            sync();
             if (valid) {
                 [[maybe_unused]] F* osq = static_cast<F*>(ob0) + obase;
                 for (int k = 1 + lt; k <= N / 2; k += T) {
@@ -1053,7 +1064,7 @@ struct TileWorker {
         }
         // The next tile's first shared-memory write is preceded by a barrier in
         // every path except the backward RFFT pre-step and the single-point case.
-        if constexpr (OP == kC2RBwd || NG == 0) __syncthreads();
+        if constexpr (OP == kC2RBwd || NG == 0) sync();
     }
 };
 
@@ -1127,7 +1138,27 @@ __global__ void __launch_bounds__(TileCfg<F, P, OP, 128, 0, NQ>::THREADS, TileCf
     const bool use_stage = Cfg::kStageBins && !GATHER && a.tma;
     if (use_stage) w.stage_bins(a, blockIdx.x);
 
+    // Where neither stages the input, L2 is asked for the next tile's while
+    // this one computes. Measured (256 MiB, us): CFFT<float> rows off 16 bytes,
+    // orders 9 / 13 / 14 213.8 -> 200.5, 377.5 -> 316.5, 389.2 -> 366.0; their RFFT
+    // forward 12 / 14 140.4 -> 115.5, 195.6 -> 164.7; RFFT<double> backward 12 / 13
+    // 143.9 -> 129.1, 166.0 -> 149.5. The shorter backward tiles lose up to 10%.
+    auto prefetch = [&](long long t) {
+        const long long tr = t * TPT + threadIdx.x;
+        if constexpr (!GATHER && (OP == kC2RBwd ? P >= 11 : P >= 8)) {
+            if (use_tma || use_stage || threadIdx.x >= TPT || tr >= a.batch) return;
+            constexpr size_t n = OP == kC2RBwd ? N + 1 : N;
+            const long long base = tr * a.in_stride;
+            if constexpr (kSoAIn) {
+                prefetch_l2(static_cast<const F*>(a.in0) + base, n * sizeof(F));
+                prefetch_l2(static_cast<const F*>(a.in1) + base, n * sizeof(F));
+            } else {
+                prefetch_l2(static_cast<const C*>(a.in0) + base, n * sizeof(C));
+            }
+        }
+    };
     for (long long tile = blockIdx.x; tile * TPT < a.batch; tile += gridDim.x) {
+        prefetch(tile + gridDim.x);
         if constexpr (Cfg::kTMA || Cfg::kTMA1) {
             if (use_tma) {
                 const bool ok = mbar_wait(bar, phase);
