@@ -323,6 +323,7 @@ struct zlfft_plan_s {
     int* d_err = nullptr;  // device error word written by kernels (bounded waits that ran out)
     // plan parameters: defaults, or the device's tuning entry for this size
     size_t chunk_mb = 48;   // scratch per chunk-pipeline buffer (measured plateau: 32-128 MiB)
+    bool chunk_tuned = false;  // chunk_mb comes from a tuning entry or ZLFFT_CHUNK_MB: used as it is
     int nlanes = 2;         // chunk pipelines
     int use_tma = 1;        // TMA staging of kernel inputs (else direct loads)
     bool tc_form = false;   // 256-point passes in the tensor-core split form
@@ -497,7 +498,10 @@ int ensure_scratch(zlfft_plan_s* p) {
     size_t budget = p->chunk_mb << 20;  // bytes of one scratch buffer
     if (const char* env = getenv("ZLFFT_CHUNK_MB")) {
         const long v = atol(env);
-        if (v > 0) budget = (size_t)v << 20;
+        if (v > 0) {
+            budget = (size_t)v << 20;
+            p->chunk_tuned = true;
+        }
     }
     size_t chunk = budget / per;
     if (chunk == 0) chunk = 1;
@@ -585,6 +589,22 @@ bool l2_discard_enabled() {
     return on;
 }
 
+// Transforms per chunk of a call: the scratch holds p->chunk per buffer (48
+// MiB by default), which a call of up to two chunks uses in full. A longer one
+// runs its two pipelines on smaller chunks: both pipelines' input, scratch and
+// output then stay in L2 together (4 x 2 x 48 MiB do not), and with launches
+// that overlap (launch_dependent) the extra ones cost little. Measured against 48 MiB:
+// 32 MiB CFFT<float> orders 15-16 +1-5%, 20-21 +5-7%, CFFT<double> 15-20 +1-10%;
+// RFFTs, whose split or pre-step is a pass of its own, 24 MiB +4-8% forward and
+// +2-7% backward at 16-19, +7-16% at 20-22. 24 MiB costs the 2-pass CFFT orders
+// 17-18 2-3%, and 16 MiB up to 9%. Gathered batches (mixed) lose 1%.
+long long call_chunk(const zlfft_plan_s* p, long long batch, bool gather) {
+    const long long c = (long long)p->chunk;
+    if (p->chunk_tuned || gather || p->nlanes < 2 || batch <= 2 * c) return c;
+    const long long s = p->kind == ZLFFT_R2C ? c / 2 : 2 * c / 3;
+    return s > 0 ? s : 1;
+}
+
 // Kernel of pass pi: the tensor-core split-precision pass where the plan asks
 // for it and one exists (256-point passes, FP32 AoS), else the plain pass.
 zlfft::PassLaunchFn pick_pass(const zlfft_plan_s* p, int pi, bool fwd, int li, int lo) {
@@ -639,7 +659,8 @@ int exec_multipass(zlfft_plan_s* p, int dop, int in_layout, int out_layout, cons
     // Chunks alternate between two internal streams forked from (and joined
     // back to) the caller's stream, so one chunk's passes overlap the other's
     // launch gaps and wave tails. Each stream owns two scratch buffers.
-    const long long nchunks = (a.batch + (long long)p->chunk - 1) / (long long)p->chunk;
+    const long long chunk = call_chunk(p, a.batch, a.gin0 != nullptr);
+    const long long nchunks = (a.batch + chunk - 1) / chunk;
     const bool fork = nchunks > 1 && p->nlanes > 1;
     if (fork) {
         if (cudaEventRecord(p->ev_fork, st) != cudaSuccess) return fail(ZLFFT_ERR_CUDA, "event record failed");
@@ -650,8 +671,8 @@ int exec_multipass(zlfft_plan_s* p, int dop, int in_layout, int out_layout, cons
     const cudaStream_t caller = st;
     const size_t quarter = p->scratch_bytes / 4;
     const bool gather = a.gin0 != nullptr;
-    for (long long b0 = 0, ci = 0; b0 < a.batch; b0 += (long long)p->chunk, ++ci) {
-        const long long nb = std::min<long long>((long long)p->chunk, a.batch - b0);
+    for (long long b0 = 0, ci = 0; b0 < a.batch; b0 += chunk, ++ci) {
+        const long long nb = std::min<long long>(chunk, a.batch - b0);
         if (fork) st = p->lanes[ci & 1];
         s0 = static_cast<char*>(p->d_scratch) + (size_t)(fork ? (ci & 1) : 0) * 2 * quarter;
         s1 = s0 + quarter;
@@ -2117,7 +2138,10 @@ int zlfft_plan_create(zlfft_plan* out, int kind, int precision, size_t order, in
     {
         TuneEntry te;
         if (tune_lookup(device, kind, precision, (int)order, &te)) {
-            if (te.chunk_mb > 0) p->chunk_mb = (size_t)te.chunk_mb;
+            if (te.chunk_mb > 0) {
+                p->chunk_mb = (size_t)te.chunk_mb;
+                p->chunk_tuned = true;
+            }
             p->nlanes = te.streams;
             p->use_tma = te.tma;
             p->fuse_split = te.split_fused != 0;
