@@ -1585,16 +1585,17 @@ struct zlfft_mixed_s {
     const void** d_gin = nullptr;
     void** d_gout = nullptr;
     zlfft::MixedGroup* d_mgroups[2] = {nullptr, nullptr};  // per precision
-    zlfft::MixedItem* d_items[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [precision][order class]
-    int n_items[2][2] = {{0, 0}, {0, 0}};
-    int* d_counter = nullptr;  // one work-list counter per (precision, order class)
+    zlfft::MixedItem* d_items[2] = {nullptr, nullptr};  // per precision
+    int n_items[2] = {0, 0};
+    int* d_counter = nullptr;  // one work-list counter per precision
     cudaStream_t cap_stream = nullptr;
     // persistent schedule: the multi-pass and large-tile groups run on these
     // streams (forked from the caller's stream, joined back) beside the
     // persistent launch
-    static constexpr int kSideStreams = 2;
-    cudaStream_t side[kSideStreams] = {nullptr, nullptr};
-    cudaEvent_t ev_fork = nullptr, ev_join[kSideStreams] = {nullptr, nullptr};
+    static constexpr int kSideStreams = 4;
+    int n_side = kSideStreams;  // those in use: two where the batch itself fills the GPU (mixed_create_impl)
+    cudaStream_t side[kSideStreams] = {};
+    cudaEvent_t ev_fork = nullptr, ev_join[kSideStreams] = {};
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
     size_t graph_launches = 0;  // kernels recorded in the graph
@@ -1713,7 +1714,7 @@ zlfft::TileArgs mixed_args(const zlfft_mixed_s* m, const MixedGroupHost& g) {
     return a;
 }
 
-bool mixed_in_persistent(const MixedGroupHost& g) { return g.P >= zlfft::kMixedMinP && g.P <= zlfft::kMixedTopP; }
+bool mixed_in_persistent(const MixedGroupHost& g) { return g.P >= zlfft::kMixedMinP && g.P <= zlfft::kMixedMaxP; }
 
 // One group as its own batched launch(es) on `st`.
 int mixed_run_group(zlfft_mixed_s* m, const MixedGroupHost& g, cudaStream_t st) {
@@ -1748,35 +1749,30 @@ int mixed_run(zlfft_mixed_s* m, int schedule, cudaStream_t st) {
     for (const MixedGroupHost& g : m->groups) big += mixed_in_persistent(g) ? 0 : 1;
     if (big) {
         ZL_CUDA(cudaEventRecord(m->ev_fork, st));
-        for (int i = 0; i < zlfft_mixed_s::kSideStreams; ++i) ZL_CUDA(cudaStreamWaitEvent(m->side[i], m->ev_fork, 0));
+        for (int i = 0; i < m->n_side; ++i) ZL_CUDA(cudaStreamWaitEvent(m->side[i], m->ev_fork, 0));
         int si = -1;
         const zlfft_plan_s* prev = nullptr;
         for (const MixedGroupHost& g : m->groups) {
             if (mixed_in_persistent(g)) continue;
             if (g.plan != prev) {
-                si = (si + 1) % zlfft_mixed_s::kSideStreams;
+                si = (si + 1) % m->n_side;
                 prev = g.plan;
             }
             int rc = mixed_run_group(m, g, m->side[si]);
             if (rc) return rc;
         }
     }
-    // the 512-thread class first: its tiles are the longest
-    for (int cls = 1; cls >= 0; --cls) {
-        for (int pr = 0; pr < 2; ++pr) {
-            if (!m->n_items[pr][cls]) continue;
-            int* ctr = m->d_counter + 2 * pr + cls;
-            ZL_CUDA(cudaMemsetAsync(ctr, 0, sizeof(int), st));
-            cudaError_t e = pr == 0 ? zlfft::launch_mixed_f32(cls, m->d_mgroups[0], m->d_items[0][cls],
-                                                              m->n_items[0][cls], ctr, st, m->num_sms)
-                                    : zlfft::launch_mixed_f64(cls, m->d_mgroups[1], m->d_items[1][cls],
-                                                              m->n_items[1][cls], ctr, st, m->num_sms);
-            if (e != cudaSuccess) return cuda_fail(e, "persistent mixed launch");
-            ++m->launches;
-        }
+    for (int pr = 0; pr < 2; ++pr) {
+        if (!m->n_items[pr]) continue;
+        int* ctr = m->d_counter + pr;
+        ZL_CUDA(cudaMemsetAsync(ctr, 0, sizeof(int), st));
+        cudaError_t e = pr == 0 ? zlfft::launch_mixed_f32(m->d_mgroups[0], m->d_items[0], m->n_items[0], ctr, st, m->num_sms)
+                                : zlfft::launch_mixed_f64(m->d_mgroups[1], m->d_items[1], m->n_items[1], ctr, st, m->num_sms);
+        if (e != cudaSuccess) return cuda_fail(e, "persistent mixed launch");
+        ++m->launches;
     }
     if (big) {
-        for (int i = 0; i < zlfft_mixed_s::kSideStreams; ++i) {
+        for (int i = 0; i < m->n_side; ++i) {
             ZL_CUDA(cudaEventRecord(m->ev_join[i], m->side[i]));
             ZL_CUDA(cudaStreamWaitEvent(st, m->ev_join[i], 0));
         }
@@ -1851,51 +1847,54 @@ int mixed_create_impl(zlfft_mixed* out, const zlfft_desc* descs, size_t n, int d
     }
     // device block: gather arrays, then per precision the group records and work lists
     std::vector<zlfft::MixedGroup> mg[2];
-    std::vector<zlfft::MixedItem> items[2][2];  // [precision][order class]
-    std::vector<long long> cost[2][2];
+    std::vector<zlfft::MixedItem> items[2];
+    std::vector<long long> cost[2];
     const size_t gin_off = 0, gout_off = n * sizeof(void*);
     size_t off = 2 * n * sizeof(void*);
     auto align_up = [](size_t v) { return (v + 255) & ~size_t{255}; };
     for (const MixedGroupHost& g : m->groups) {
         if (!mixed_in_persistent(g)) continue;
         const int pr = g.prec == ZLFFT_F32 ? 0 : 1;
-        const int cls = zlfft::mixed_class(g.P);
         const int tpc = zlfft::mixed_tpc(g.P);
         const long long tiles = ((long long)g.count + tpc - 1) / tpc;
         for (long long t = 0; t < tiles; ++t) {
-            items[pr][cls].push_back(zlfft::MixedItem{(int)mg[pr].size(), (int)t});
-            cost[pr][cls].push_back(mixed_tile_cost(g.P));
+            items[pr].push_back(zlfft::MixedItem{(int)mg[pr].size(), (int)t});
+            cost[pr].push_back(mixed_tile_cost(g.P));
         }
         mg[pr].push_back(zlfft::MixedGroup{zlfft::TileArgs{}, zlfft::mixed_code(g.dop, g.P)});
     }
     for (int pr = 0; pr < 2; ++pr) {
-        for (int cls = 0; cls < 2; ++cls) {
-            // longest tiles first (groups are already in descending order; keep it stable)
-            std::vector<zlfft::MixedItem>& it = items[pr][cls];
-            std::vector<size_t> o(it.size());
-            for (size_t i = 0; i < o.size(); ++i) o[i] = i;
-            std::stable_sort(o.begin(), o.end(),
-                             [&](size_t x, size_t y) { return cost[pr][cls][x] > cost[pr][cls][y]; });
-            std::vector<zlfft::MixedItem> sorted(o.size());
-            for (size_t i = 0; i < o.size(); ++i) sorted[i] = it[o[i]];
-            it.swap(sorted);
-            if (it.size() > (size_t)INT32_MAX) {
-                mixed_release(m);
-                return fail(ZLFFT_ERR_INVALID_ARG, "too many tiles");
-            }
-            m->n_items[pr][cls] = (int)it.size();
+        // longest tiles first (groups are already in descending order; keep it stable)
+        std::vector<zlfft::MixedItem>& it = items[pr];
+        std::vector<size_t> o(it.size());
+        for (size_t i = 0; i < o.size(); ++i) o[i] = i;
+        std::stable_sort(o.begin(), o.end(), [&](size_t x, size_t y) { return cost[pr][x] > cost[pr][y]; });
+        std::vector<zlfft::MixedItem> sorted(o.size());
+        for (size_t i = 0; i < o.size(); ++i) sorted[i] = it[o[i]];
+        it.swap(sorted);
+        if (it.size() > (size_t)INT32_MAX) {
+            mixed_release(m);
+            return fail(ZLFFT_ERR_INVALID_ARG, "too many tiles");
         }
+        m->n_items[pr] = (int)it.size();
     }
-    size_t grp_off[2], item_off[2][2];
+    // Side streams in use. Four overlap the many short launches of a small batch
+    // (us, two -> four streams: 60 transforms of orders 6-16 39.1 -> 24.7, 300 of
+    // 10-14 34.7 -> 22.8, 1000 of 10-16 131 -> 116); a batch of gigabytes loses to
+    // the extra scratch in L2 (20,000 of 6-16, 2.8 GB: 1120 -> 1139).
+    {
+        size_t bytes = 0;  // read and written
+        for (const MixedGroupHost& g : m->groups) bytes += g.count * (size_t{1} << g.P) * (g.prec == ZLFFT_F32 ? 16 : 32);
+        m->n_side = bytes > (size_t{1} << 30) ? 2 : zlfft_mixed_s::kSideStreams;
+    }
+    size_t grp_off[2], item_off[2];
     for (int pr = 0; pr < 2; ++pr) {
         off = align_up(off);
         grp_off[pr] = off;
         off += mg[pr].size() * sizeof(zlfft::MixedGroup);
-        for (int cls = 0; cls < 2; ++cls) {
-            off = align_up(off);
-            item_off[pr][cls] = off;
-            off += items[pr][cls].size() * sizeof(zlfft::MixedItem);
-        }
+        off = align_up(off);
+        item_off[pr] = off;
+        off += items[pr].size() * sizeof(zlfft::MixedItem);
     }
     // Multi-pass groups: one tensor map per transform for the first pass's bulk
     // copies (the contiguous path's single map cannot describe scattered
@@ -1931,7 +1930,7 @@ int mixed_create_impl(zlfft_mixed* out, const zlfft_desc* descs, size_t n, int d
     off += h_maps.size() * sizeof(CUtensorMap);
     off = align_up(off);
     const size_t counter_off = off;
-    off += 4 * sizeof(int);
+    off += 2 * sizeof(int);
     if (cudaMalloc(&m->d_mem, off) != cudaSuccess) {
         cudaGetLastError();
         mixed_release(m);
@@ -1963,16 +1962,14 @@ int mixed_create_impl(zlfft_mixed* out, const zlfft_desc* descs, size_t n, int d
         if (!mg[pr].empty())
             e = cudaMemcpy(m->d_mgroups[pr], mg[pr].data(), mg[pr].size() * sizeof(zlfft::MixedGroup),
                            cudaMemcpyHostToDevice);
-        for (int cls = 0; cls < 2 && e == cudaSuccess; ++cls) {
-            m->d_items[pr][cls] = reinterpret_cast<zlfft::MixedItem*>(base + item_off[pr][cls]);
-            if (!items[pr][cls].empty())
-                e = cudaMemcpy(m->d_items[pr][cls], items[pr][cls].data(),
-                               items[pr][cls].size() * sizeof(zlfft::MixedItem), cudaMemcpyHostToDevice);
-        }
+        m->d_items[pr] = reinterpret_cast<zlfft::MixedItem*>(base + item_off[pr]);
+        if (e == cudaSuccess && !items[pr].empty())
+            e = cudaMemcpy(m->d_items[pr], items[pr].data(), items[pr].size() * sizeof(zlfft::MixedItem),
+                           cudaMemcpyHostToDevice);
     }
     if (e == cudaSuccess && !h_maps.empty())
         e = cudaMemcpy(base + maps_off, h_maps.data(), h_maps.size() * sizeof(CUtensorMap), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemset(m->d_counter, 0, 4 * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemset(m->d_counter, 0, 2 * sizeof(int));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->cap_stream, cudaStreamNonBlocking);
     for (int i = 0; i < zlfft_mixed_s::kSideStreams && e == cudaSuccess; ++i) {
         e = cudaStreamCreateWithFlags(&m->side[i], cudaStreamNonBlocking);
