@@ -115,9 +115,8 @@ cudaError_t launch_tile_gather(const TileArgs& a, cudaStream_t stream, const Lau
     const long long tiles = (a.batch + Cfg::TPT - 1) / Cfg::TPT;
     const long long cap = (long long)ctx.num_sms * blocks_per_sm;
     const unsigned grid = (unsigned)(tiles < cap ? tiles : cap);
-    kern<<<grid, Cfg::THREADS, Tabs::SMEM, stream>>>(a);
     if (ctx.launches) ++*ctx.launches;
-    return cudaGetLastError();
+    return launch_dependent(kern, grid, Cfg::THREADS, Tabs::SMEM, stream, a);
 }
 
 template <typename F, int P>
