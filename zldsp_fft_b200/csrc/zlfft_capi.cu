@@ -597,10 +597,11 @@ bool l2_discard_enabled() {
 // 32 MiB CFFT<float> orders 15-16 +1-5%, 20-21 +5-7%, CFFT<double> 15-20 +1-10%;
 // RFFTs, whose split or pre-step is a pass of its own, 24 MiB +4-8% forward and
 // +2-7% backward at 16-19, +7-16% at 20-22. 24 MiB costs the 2-pass CFFT orders
-// 17-18 2-3%, and 16 MiB up to 9%. Gathered batches (mixed) lose 1%.
+// 17-18 2-3%, and 16 MiB up to 9%. Gathered batches (mixed) lose 1%, the
+// tensor-core form (whose launches do not overlap) 2-4%: both keep 48 MiB.
 long long call_chunk(const zlfft_plan_s* p, long long batch, bool gather) {
     const long long c = (long long)p->chunk;
-    if (p->chunk_tuned || gather || p->nlanes < 2 || batch <= 2 * c) return c;
+    if (p->chunk_tuned || p->tc_form || gather || p->nlanes < 2 || batch <= 2 * c) return c;
     const long long s = p->kind == ZLFFT_R2C ? c / 2 : 2 * c / 3;
     return s > 0 ? s : 1;
 }

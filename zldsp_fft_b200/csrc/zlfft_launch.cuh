@@ -50,7 +50,8 @@ cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, int threads, size_t 
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+    return e == cudaSuccess ? cudaSuccess : cudaGetLastError();  // (reported once, as after a <<<>>> launch)
 }
 
 using TileLaunchFn = cudaError_t (*)(const TileArgs&, cudaStream_t, const LaunchCtx&);

@@ -13,7 +13,10 @@
 // when the count of remaining radix-4 stages is odd, then radix-16 groups.
 // The last group is therefore radix-16 with one butterfly per thread, and
 // its twiddles depend on the thread only: they are loaded into registers
-// once per CTA and reused for every transform the CTA processes.
+// once per CTA and reused for every transform the CTA processes. The other
+// groups' twiddles, the RFFT split twiddles and the STFT window are read from
+// copies in shared memory (TileTabs). Some kernels run NQ = 2 transforms per
+// thread, which share those reads (tile_nq, zlfft_launch.cuh).
 //
 // The RFFT epilogue of the reference (execute.hpp:318-368 forward split,
 // :481-536 squared magnitude) is fused after the last group without another
@@ -204,7 +207,8 @@ struct TileCfg {
     static constexpr bool kStageBins = OP == kC2RBwd && sizeof(F) == 4 && (P == 9 || (P >= 11 && P <= 13)) &&
                                        XBYTES + BBYTES <= 200 * 1024;
     // 128 KB tiles (FP32 order 14, FP64 order 13: no room for a second
-    // buffer): the next tile's input lands by TMA in the exchange buffer
+    // buffer) and tiles of two transforms per thread (a second buffer would
+    // cost resident CTAs): the next tile's input lands by TMA in the exchange buffer
     // itself, once the last group has read it, while the last group computes
     // and stores. For the forward RFFT only where the split runs in registers
     // (the shuffle epilogue of TileWorker: last group radix 16 = E), so the
