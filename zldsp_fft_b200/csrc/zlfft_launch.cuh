@@ -73,12 +73,13 @@ struct TileTable {
 // registers (4 CTAs of 128 threads per SM instead of 5, with twice the
 // transforms in flight) and the separate staging buffer. Measured, complex
 // orders 9-11 (us, one -> two): STFT squared magnitudes 195.9 -> 182.1, 203.2 ->
-// 186.1, 208.2 -> 183.6; batched squared magnitudes at 10 and 11 102.0 -> 97.2,
-// 102.4 -> 97.6. The forward bins gain nothing (bound by their stores), and
-// from order 12 on the CTAs grow too large (order 13 106.0 -> 112.5).
+// 186.1, 208.2 -> 183.6; batched squared magnitudes 98.5 -> 92.5, 102.0 -> 97.2,
+// 102.4 -> 97.6; forward bins 96.7 -> 97.9 (split re/im 102.0 -> 110.2), 102.2 ->
+// 104.4, 108.3 -> 108.7 (bound by their stores); CFFTs 175.5 -> 191.7, 185.6 -> 194.8; and
+// from order 12 on the CTAs grow too large (squared magnitudes 106.0 -> 112.5).
 template <typename F, int P, int OP, bool WIN, bool FAST>
 constexpr int tile_nq() {
-    return sizeof(F) == 4 && P <= 11 && ((WIN && P >= 9) || (OP == kR2CSqrMag && P >= 10)) ? 2 : 1;
+    return sizeof(F) == 4 && P >= 9 && P <= 11 && (WIN || OP == kR2CSqrMag) ? 2 : 1;
 }
 
 template <typename F, int P, int OP, int IL, int OL, bool WIN = false, bool FAST = false>
