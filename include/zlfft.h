@@ -327,9 +327,10 @@ ZLFFT_API int zlfft_exec_mixed_device(const zlfft_desc* descs, size_t n, void* s
  * afterwards on that device and size uses the tuned chunk, pipelines and
  * staging; plans created with ZLFFT_MODE_TUNED also take the tuned form
  * (without a tuning entry they behave as ZLFFT_MODE_PLAIN). Mixed batches
- * create their plans with ZLFFT_MODE_TUNED. If the environment variable
- * ZLFFT_TUNE_FILE names a file written by zlfft_tuning_save, the first plan
- * created on a device loads it. */
+ * create their plans with ZLFFT_MODE_TUNED, and run complex orders up to 13 in
+ * the plain form whatever the entry says (one form for every schedule). If the
+ * environment variable ZLFFT_TUNE_FILE names a file written by
+ * zlfft_tuning_save, the first plan created on a device loads it. */
 typedef struct zlfft_tuning {
     int chunk_mb;       /* scratch per chunk pipeline buffer, MiB (0: single-tile size) */
     int streams;        /* chunk pipelines, 1 or 2 */

@@ -1559,11 +1559,12 @@ int exec_host_impl(zlfft_plan_s* p, int op, int in_layout, int out_layout, const
 // A mixed batch is sorted on the host into groups of one (precision, kind,
 // order, operation); each group's transforms are addressed through gathered
 // pointer arrays (transform t of the group reads gin[t], writes gout[t]).
-// Groups of complex order 2..13 become tiles of persistent launches, one per
-// (precision, order class): orders 2..11 in 128-thread CTAs, 12..13 in
-// 512-thread CTAs (zlfft_mixed.cuh); the others run as gathered batched
-// launches of the tile kernel (orders 0, 1 and the FP32 order-14 tile) or of
-// the multi-pass pipeline (14 and up), largest first.
+// Groups of complex order 2..11 become tiles of one persistent launch per
+// precision (zlfft_mixed.cuh); the others run as gathered batched launches of
+// the tile kernel (orders 0, 1, 12, 13 and the FP32 order-14 tile) or of the
+// multi-pass pipeline (14 and up), largest first. Every schedule gives the
+// same bits: complex orders up to 13 always run in the plain form, larger ones
+// in the tuned plan's.
 struct MixedGroupHost {
     zlfft_plan plan;
     int prec;
@@ -1725,7 +1726,9 @@ int mixed_run_group(zlfft_mixed_s* m, const MixedGroupHost& g, cudaStream_t st) 
         return exec_multipass(g.plan, g.dop, ZLFFT_AOS, ZLFFT_AOS, a, st, ctx);
     const zlfft::GatherTable& t = g.prec == ZLFFT_F32 ? tables().g32 : tables().g64;
     zlfft::TileLaunchFn fn = t.fn[g.P][g.dop];
-    if (g.plan->fast_form && t.fast[g.P][g.dop]) fn = t.fast[g.P][g.dop];  // the tuned plan's form
+    // the tuned plan's form, for the order-14 tile alone: orders up to 13 are plain in every schedule,
+    // as the persistent kernel runs them
+    if (g.plan->fast_form && t.fast[g.P][g.dop]) fn = t.fast[g.P][g.dop];
     if (!fn) return fail(ZLFFT_ERR_UNSUPPORTED, "no gathered kernel for order %d", g.P);
     cudaError_t e = fn(a, st, ctx);
     if (e != cudaSuccess) return cuda_fail(e, "gathered tile launch");

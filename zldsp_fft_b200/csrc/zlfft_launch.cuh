@@ -103,7 +103,7 @@ cudaError_t launch_tile(const TileArgs& a, cudaStream_t stream, const LaunchCtx&
 // the AoS <-> AoS operations: [order][op].
 struct GatherTable {
     TileLaunchFn fn[kTileTableP + 1][5];
-    TileLaunchFn fast[kTileTableP + 1][5];  // the fast-twiddle form, orders 11 and up (not C2R)
+    TileLaunchFn fast[kTileTableP + 1][5];  // the fast-twiddle form, order 14 (not C2R)
 };
 
 template <typename F, int P, int OP, bool FAST = false>
@@ -123,7 +123,7 @@ cudaError_t launch_tile_gather(const TileArgs& a, cudaStream_t stream, const Lau
 
 template <typename F, int P>
 void fill_gather_fast(GatherTable& t) {
-    if constexpr (P >= 11) {
+    if constexpr (P >= 14) {
         t.fast[P][kC2CFwd] = launch_tile_gather<F, P, kC2CFwd, true>;
         t.fast[P][kC2CBwd] = launch_tile_gather<F, P, kC2CBwd, true>;
         t.fast[P][kR2CFwd] = launch_tile_gather<F, P, kR2CFwd, true>;
