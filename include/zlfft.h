@@ -332,14 +332,14 @@ ZLFFT_API int zlfft_exec_mixed_device(const zlfft_desc* descs, size_t n, void* s
  * environment variable ZLFFT_TUNE_FILE names a file written by
  * zlfft_tuning_save, the first plan created on a device loads it. */
 typedef struct zlfft_tuning {
-    int chunk_mb;       /* scratch per chunk pipeline buffer, MiB (0: single-tile size) */
+    int chunk_mb;       /* scratch per chunk pipeline buffer, MiB (0: the default's rule, by the size of each call) */
     int streams;        /* chunk pipelines, 1 or 2 */
     int tma;            /* 1: inputs staged by TMA copies; 0: direct loads */
     int form;           /* ZLFFT_MODE_PLAIN, ZLFFT_MODE_FAST or ZLFFT_MODE_TC_FP16 */
     int split_fused;    /* RFFT forward: 1 = split fused into the last pass, 0 = its own kernel */
     int store_tma;      /* first pass: 1 = output by TMA tensor stores, 0 = copied out, -1 = default */
     double gbs;         /* measured algorithmic GB/s of the chosen plan (forward, AoS) */
-    double gbs_default; /* of the default plan (48 MiB, 2 pipelines, TMA, plain) */
+    double gbs_default; /* of the default plan (2 pipelines, TMA, plain) */
 } zlfft_tuning;
 
 /* Measure the candidate plans of every order in [order_lo, order_hi] for
@@ -358,6 +358,12 @@ ZLFFT_API int zlfft_tuning_get(int device, int kind, int precision, size_t order
  * another name or SM count are skipped). *loaded = entries taken. */
 ZLFFT_API int zlfft_tuning_save(int device, const char* path);
 ZLFFT_API int zlfft_tuning_load(int device, const char* path, size_t* loaded);
+
+/* Autotuner self-test: the kernels that one call (forward, AoS, `batch`
+ * transforms) launches when the autotuner times `entry`, whatever the table
+ * holds for the size: those of a plan made from that entry. */
+ZLFFT_API int zlfft_selftest_tune_launches(int device, int kind, int precision, size_t order, const zlfft_tuning* entry,
+                                           size_t batch, size_t* launches);
 
 /* Forget every tuning entry of every device. */
 ZLFFT_API int zlfft_tuning_clear(void);

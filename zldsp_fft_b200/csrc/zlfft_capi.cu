@@ -2095,11 +2095,12 @@ int apply_switch(zlfft_plan_s* p, int max_l1_order, int switch_order) {
     return ZLFFT_OK;
 }
 
-}  // namespace
-
-extern "C" {
-
-int zlfft_plan_create(zlfft_plan* out, int kind, int precision, size_t order, int mode, int device) {
+// zlfft_plan_create with the parameters of `entry` in place of the device's
+// tuning entry for the size (null: the device's entry, if it has one). The
+// autotuner makes its candidates here, so what it times is what a plan made
+// from the recorded entry runs.
+int plan_create_impl(zlfft_plan* out, int kind, int precision, size_t order, int mode, int device,
+                     const TuneEntry* entry) {
     if (!out) return fail(ZLFFT_ERR_INVALID_ARG, "plan pointer is null");
     *out = nullptr;
     if (kind != ZLFFT_C2C && kind != ZLFFT_R2C) return fail(ZLFFT_ERR_INVALID_ARG, "invalid kind %d", kind);
@@ -2138,8 +2139,13 @@ int zlfft_plan_create(zlfft_plan* out, int kind, int precision, size_t order, in
     }
     {
         TuneEntry te;
-        if (tune_lookup(device, kind, precision, (int)order, &te)) {
-            if (te.chunk_mb > 0) {
+        bool have = entry != nullptr;
+        if (have)
+            te = *entry;
+        else
+            have = tune_lookup(device, kind, precision, (int)order, &te);
+        if (have) {
+            if (te.chunk_mb > 0) {  // (0: the rule of call_chunk)
                 p->chunk_mb = (size_t)te.chunk_mb;
                 p->chunk_tuned = true;
             }
@@ -2260,6 +2266,14 @@ int zlfft_plan_create(zlfft_plan* out, int kind, int precision, size_t order, in
     }
     *out = p;
     return ZLFFT_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int zlfft_plan_create(zlfft_plan* out, int kind, int precision, size_t order, int mode, int device) {
+    return plan_create_impl(out, kind, precision, order, mode, device, nullptr);
 }
 
 int zlfft_plan_create_hybrid(zlfft_plan* out, int kind, int precision, size_t order, int max_l1_order,
@@ -2486,17 +2500,13 @@ const char* zlfft_version(void) { return "zlfft-b200 0.1 (sm_100a)"; }
 
 namespace {
 
-// One candidate plan timed on `batch` transforms: forward AoS -> AoS.
+// One candidate plan timed on `batch` transforms: forward AoS -> AoS. *launches
+// (may be null): the kernels of one call.
 int time_candidate(int device, int kind, int prec, int order, const TuneEntry& c, const void* in, void* out,
-                   size_t batch, cudaStream_t st, double* ms) {
+                   size_t batch, cudaStream_t st, double* ms, size_t* launches = nullptr) {
     zlfft_plan p = nullptr;
-    int rc = zlfft_plan_create(&p, kind, prec, (size_t)order, c.form, device);
+    int rc = plan_create_impl(&p, kind, prec, (size_t)order, ZLFFT_MODE_TUNED, device, &c);
     if (rc) return rc;
-    p->chunk_mb = c.chunk_mb > 0 ? (size_t)c.chunk_mb : p->chunk_mb;
-    p->nlanes = c.streams;
-    p->use_tma = c.tma;
-    p->fuse_split = c.split_fused != 0;
-    p->store_tma = c.store_tma;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -2516,6 +2526,7 @@ int time_candidate(int device, int kind, int prec, int order, const TuneEntry& c
     cudaEventDestroy(e1);
     int st_err = 0;
     cudaMemcpy(&st_err, p->d_err, sizeof(int), cudaMemcpyDeviceToHost);
+    if (launches) *launches = p->launches / (kReps + 2);
     release(p);
     if (rc) return rc;
     if (e != cudaSuccess) return cuda_fail(e, "autotune timing");
@@ -2558,15 +2569,18 @@ int autotune_impl(int device, int kind, int prec, size_t lo, size_t hi) {
         const size_t batch = std::max<size_t>(1, budget / std::max(per_in, per_out));
         std::vector<TuneEntry> cands;
         const bool tc_ok = kind == ZLFFT_C2C && prec == ZLFFT_F32 && cfft_order >= zlfft::kPassMinP;
+        const bool one_tile = cfft_order == 14 && prec == ZLFFT_F32;  // no chunks but in the tensor-core form (tile14)
         if (cfft_order >= zlfft::kPassMinP) {
             for (int form : {ZLFFT_MODE_PLAIN, ZLFFT_MODE_FAST, ZLFFT_MODE_TC_FP16}) {
                 if (form == ZLFFT_MODE_TC_FP16 && !tc_ok) continue;
-                for (int chunk : {16, 32, 48, 96, 192})
+                // chunk 0 is the default's rule (call_chunk), where it is not 48 MiB
+                for (int chunk : {0, 16, 32, 48, 96, 192})
                     for (int streams : {1, 2})
                         for (int tma : {0, 1})
                             for (int fused : {0, 1})
                                 for (int store : {0, 1}) {
                                     if (fused && kind != ZLFFT_R2C) continue;
+                                    if (chunk == 0 && (form == ZLFFT_MODE_TC_FP16 || one_tile || streams == 1)) continue;
                                     TuneEntry c;
                                     c.chunk_mb = chunk;
                                     c.streams = streams;
@@ -2599,8 +2613,8 @@ int autotune_impl(int device, int kind, int prec, size_t lo, size_t hi) {
             const double gbs = (double)batch * (double)(per_in + per_out) / (ms * 1e6);
             const int store_default = prec == ZLFFT_F32 ? 1 : 0;
             const bool is_default = c.form == ZLFFT_MODE_PLAIN && c.tma == 1 && c.split_fused == 0 &&
-                                    (c.chunk_mb == 0 || (c.chunk_mb == 48 && c.streams == 2 &&
-                                                         c.store_tma == store_default));
+                                    (cfft_order < zlfft::kPassMinP ||
+                                     (c.chunk_mb == (one_tile ? 48 : 0) && c.streams == 2 && c.store_tma == store_default));
             if (is_default) def_gbs = gbs;
             if (gbs > best_gbs) {
                 best_gbs = gbs;
@@ -2625,6 +2639,43 @@ extern "C" {
 
 int zlfft_autotune(int device, int kind, int precision, size_t order_lo, size_t order_hi) {
     return autotune_impl(device, kind, precision, order_lo, order_hi);
+}
+
+int zlfft_selftest_tune_launches(int device, int kind, int precision, size_t order, const zlfft_tuning* entry,
+                                 size_t batch, size_t* launches) {
+    if (!entry || !launches) return fail(ZLFFT_ERR_INVALID_ARG, "null argument");
+    if (order > 24 || batch == 0) return fail(ZLFFT_ERR_INVALID_ARG, "order or batch out of range");
+    if (entry->form == ZLFFT_MODE_TC_FP16 && (kind != ZLFFT_C2C || precision != ZLFFT_F32))
+        return fail(ZLFFT_ERR_UNSUPPORTED, "the tensor-core split form is built for CFFT<float>");
+    if (device < 0 && cudaGetDevice(&device) != cudaSuccess) return fail(ZLFFT_ERR_CUDA, "no CUDA device");
+    DeviceGuard g(device);
+    TuneEntry c;
+    c.chunk_mb = entry->chunk_mb;
+    c.streams = entry->streams;
+    c.tma = entry->tma;
+    c.form = entry->form;
+    c.split_fused = entry->split_fused;
+    c.store_tma = entry->store_tma;
+    const size_t bytes = batch * ((size_t{1} << order) + 2) * 2 * (precision == ZLFFT_F32 ? 4 : 8);
+    void* d = nullptr;
+    if (cudaMalloc(&d, 2 * bytes) != cudaSuccess) {
+        cudaGetLastError();
+        return alloc_fail("self-test", 2 * bytes);
+    }
+    cudaStream_t st = nullptr;
+    double ms = 0;
+    int rc = ZLFFT_OK;
+    cudaError_t e = cudaMemset(d, 0, 2 * bytes);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (e != cudaSuccess)
+        rc = cuda_fail(e, "tuning self-test");
+    else
+        rc = time_candidate(device, kind, precision, (int)order, c, d, static_cast<char*>(d) + bytes, batch, st, &ms,
+                            launches);
+    if (st) cudaStreamDestroy(st);
+    cudaFree(d);
+    return rc;
 }
 
 int zlfft_tuning_get(int device, int kind, int precision, size_t order, zlfft_tuning* out) {
