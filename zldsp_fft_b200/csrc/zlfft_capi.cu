@@ -542,6 +542,14 @@ dim3 pair_grid(const zlfft_plan_s* p, int M, long long batch) {
     return dim3((unsigned)gx, (unsigned)gy, 1);
 }
 
+// Whether the CTAs of the size's first pass take an SM each (FP64 passes of 512
+// and 1024 points: 145 KB).
+template <typename F>
+bool first_pass_fills_sm(const zlfft_plan_s* p) {
+    static_assert(zlfft::PassCfg<double, 17, 0>::MINB == 1 && zlfft::PassCfg<double, 18, 0>::MINB == 1);
+    return sizeof(F) == 8 && (p->cfft_order == 17 || p->cfft_order == 18);
+}
+
 template <typename F>
 cudaError_t launch_split(const zlfft_plan_s* p, int dop, int out_layout, const void* z, void* o0, void* o1,
                          long long batch, long long out_stride, cudaStream_t st, const zlfft::LaunchCtx& ctx,
@@ -551,13 +559,14 @@ cudaError_t launch_split(const zlfft_plan_s* p, int dop, int out_layout, const v
     const dim3 grid = pair_grid(p, M, batch);
     const C* zc = static_cast<const C*>(z);
     const C* rw = static_cast<const C*>(p->d_rw);
+    const int early = ctx.beside || first_pass_fills_sm<F>(p) ? 1 : 0;
     cudaError_t e;
     if (dop == zlfft::kR2CSqrMag)
-        e = zlfft::launch_dependent(zlfft::rfft_split_kernel<F, zlfft::kR2CSqrMag, zlfft::kAoS>, grid, 256, 0, st, zc, o0, o1, rw, M, batch, M, out_stride, go0, go1);
+        e = zlfft::launch_dependent(zlfft::rfft_split_kernel<F, zlfft::kR2CSqrMag, zlfft::kAoS>, grid, 256, 0, st, zc, o0, o1, rw, M, batch, M, out_stride, go0, go1, early);
     else if (out_layout == ZLFFT_AOS)
-        e = zlfft::launch_dependent(zlfft::rfft_split_kernel<F, zlfft::kR2CFwd, zlfft::kAoS>, grid, 256, 0, st, zc, o0, o1, rw, M, batch, M, out_stride, go0, go1);
+        e = zlfft::launch_dependent(zlfft::rfft_split_kernel<F, zlfft::kR2CFwd, zlfft::kAoS>, grid, 256, 0, st, zc, o0, o1, rw, M, batch, M, out_stride, go0, go1, early);
     else
-        e = zlfft::launch_dependent(zlfft::rfft_split_kernel<F, zlfft::kR2CFwd, zlfft::kSoA>, grid, 256, 0, st, zc, o0, o1, rw, M, batch, M, out_stride, go0, go1);
+        e = zlfft::launch_dependent(zlfft::rfft_split_kernel<F, zlfft::kR2CFwd, zlfft::kSoA>, grid, 256, 0, st, zc, o0, o1, rw, M, batch, M, out_stride, go0, go1, early);
     if (ctx.launches) ++*ctx.launches;
     return e;
 }
@@ -570,11 +579,12 @@ cudaError_t launch_pre(const zlfft_plan_s* p, int in_layout, const void* i0, con
     const int M = 1 << p->cfft_order;
     const dim3 grid = pair_grid(p, M, batch);
     const C* rw = static_cast<const C*>(p->d_rw);
+    const int early = ctx.beside || first_pass_fills_sm<F>(p) ? 1 : 0;
     cudaError_t e;
     if (in_layout == ZLFFT_AOS)
-        e = zlfft::launch_dependent(zlfft::rfft_pre_kernel<F, zlfft::kAoS>, grid, 256, 0, st, i0, i1, static_cast<C*>(z), rw, M, batch, in_stride, M, gi0, gi1);
+        e = zlfft::launch_dependent(zlfft::rfft_pre_kernel<F, zlfft::kAoS>, grid, 256, 0, st, i0, i1, static_cast<C*>(z), rw, M, batch, in_stride, M, gi0, gi1, early);
     else
-        e = zlfft::launch_dependent(zlfft::rfft_pre_kernel<F, zlfft::kSoA>, grid, 256, 0, st, i0, i1, static_cast<C*>(z), rw, M, batch, in_stride, M, gi0, gi1);
+        e = zlfft::launch_dependent(zlfft::rfft_pre_kernel<F, zlfft::kSoA>, grid, 256, 0, st, i0, i1, static_cast<C*>(z), rw, M, batch, in_stride, M, gi0, gi1, early);
     if (ctx.launches) ++*ctx.launches;
     return e;
 }
@@ -636,7 +646,7 @@ zlfft::PassLaunchFn pick_pass(const zlfft_plan_s* p, int pi, bool fwd, int li, i
 // pre-step (backward) as a separate elementwise kernel on the N/2-point
 // spectrum, with the reference's arithmetic.
 int exec_multipass(zlfft_plan_s* p, int dop, int in_layout, int out_layout, const zlfft::TileArgs& a,
-                   cudaStream_t st, const zlfft::LaunchCtx& ctx) {
+                   cudaStream_t st, const zlfft::LaunchCtx& call_ctx) {
     const int P = p->cfft_order;
     if (P < zlfft::kPassMinP || P > zlfft::kPassMaxP)
         return fail(ZLFFT_ERR_UNSUPPORTED, "order %d is above the supported maximum", p->order);
@@ -663,6 +673,8 @@ int exec_multipass(zlfft_plan_s* p, int dop, int in_layout, int out_layout, cons
     const long long chunk = call_chunk(p, a.batch, a.gin0 != nullptr);
     const long long nchunks = (a.batch + chunk - 1) / chunk;
     const bool fork = nchunks > 1 && p->nlanes > 1;
+    zlfft::LaunchCtx ctx = call_ctx;
+    ctx.beside |= fork;
     if (fork) {
         if (cudaEventRecord(p->ev_fork, st) != cudaSuccess) return fail(ZLFFT_ERR_CUDA, "event record failed");
         for (int i = 0; i < 2; ++i)
@@ -1719,8 +1731,8 @@ zlfft::TileArgs mixed_args(const zlfft_mixed_s* m, const MixedGroupHost& g) {
 bool mixed_in_persistent(const MixedGroupHost& g) { return g.P >= zlfft::kMixedMinP && g.P <= zlfft::kMixedMaxP; }
 
 // One group as its own batched launch(es) on `st`.
-int mixed_run_group(zlfft_mixed_s* m, const MixedGroupHost& g, cudaStream_t st) {
-    zlfft::LaunchCtx ctx{m->num_sms, &m->launches};
+int mixed_run_group(zlfft_mixed_s* m, const MixedGroupHost& g, cudaStream_t st, bool beside) {
+    zlfft::LaunchCtx ctx{m->num_sms, &m->launches, beside};
     const zlfft::TileArgs a = mixed_args(m, g);
     if (g.P > zlfft::kTileMaxP && !tile14(g.plan))
         return exec_multipass(g.plan, g.dop, ZLFFT_AOS, ZLFFT_AOS, a, st, ctx);
@@ -1739,7 +1751,7 @@ int mixed_run(zlfft_mixed_s* m, int schedule, cudaStream_t st) {
     const bool persistent = schedule != ZLFFT_SCHED_PER_ORDER;
     if (!persistent) {  // the baseline: one batched launch (or pipeline) per group, in order
         for (const MixedGroupHost& g : m->groups) {
-            int rc = mixed_run_group(m, g, st);
+            int rc = mixed_run_group(m, g, st, false);
             if (rc) return rc;
         }
         return ZLFFT_OK;
@@ -1762,7 +1774,7 @@ int mixed_run(zlfft_mixed_s* m, int schedule, cudaStream_t st) {
                 si = (si + 1) % m->n_side;
                 prev = g.plan;
             }
-            int rc = mixed_run_group(m, g, m->side[si]);
+            int rc = mixed_run_group(m, g, m->side[si], true);
             if (rc) return rc;
         }
     }

@@ -302,6 +302,12 @@ __device__ __forceinline__ void discard_l2_line(const void* p) {
 // are visible. Every thread calls pdl_wait before it touches the caller's
 // buffers or scratch; only the plan's own tables, written before the plan
 // was handed out, may be read ahead of it. Both are no-ops in a plain launch.
+//
+// pdl_trigger comes after pdl_wait, so that one kernel at a time waits beside
+// the one that runs. Triggered before it, kernel after kernel of a chain took
+// up slots to wait in, and the CTAs of each were placed in what was left, unevenly: a
+// CFFT<float> of order 19 by itself took 15.8 us a call in a chain of calls, against 8.7
+// (10.2 without overlap); 1184 of order 9 5.1 against 3.6.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

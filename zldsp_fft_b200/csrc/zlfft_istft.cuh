@@ -124,8 +124,8 @@ __global__ void __launch_bounds__(IstftCfg<F, P>::THREADS, 1) istft_kernel(const
     const long long hp = o.hop / 2;  // hop in sample pairs
     const C zero = cx<C>((F)0, (F)0);
     for (int i = lt; i < N; i += T) ring[i] = zero;
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();
     const long long m0 = ((long long)grp * gridDim.x + blockIdx.x) * o.run;
     const long long m1 = (m0 + o.run < o.blocks) ? m0 + o.run : o.blocks;
     const long long f0 = (m0 - o.k + 1 > 0) ? m0 - o.k + 1 : 0;

@@ -364,8 +364,8 @@ __global__ void __launch_bounds__(PassCfg<F, P, PI, S>::THREADS, PassCfg<F, P, P
         twl = t;
         __syncthreads();
     }
-    pdl_trigger();
     pdl_wait();
+    pdl_trigger();
     if constexpr (Cfg::kTMA) issue(blockIdx.x);
     uint32_t phase = 0;
 
@@ -729,15 +729,24 @@ __global__ void __launch_bounds__(PassCfg<F, P, PI, S>::THREADS, PassCfg<F, P, P
 // One thread per bin pair (k, M - k), k = 0 .. M/2 (k = 0 is DC/Nyquist):
 // grid x covers the pairs of a transform, grid y strides over the transforms
 // (no 64-bit division per element).
+//
+// The kernel after them is a pass, and it begins when they are done unless
+// `early` lets it in before: their many short CTAs leave slots unevenly, and a
+// pass placed among them runs unevenly (RFFT<float> of order 19, two
+// transforms: forward 14.4 us a call against 11.7). `early` is for calls with two
+// chunks at work, and for first passes whose CTAs take an SM each, where there
+// is nothing to place unevenly (RFFT<double> of order 18, eight transforms: 21.9
+// us against 25.3).
 template <typename F, int OP, int LAYOUT>
 __global__ void rfft_split_kernel(const Cx<F>* z, void* out0, void* out1, const Cx<F>* rw, int M, long long batch,
-                                  long long z_stride, long long out_stride, void* const* gout0, void* const* gout1) {
+                                  long long z_stride, long long out_stride, void* const* gout0, void* const* gout1,
+                                  int early) {
     using C = Cx<F>;
     const int k = (int)(blockIdx.x * blockDim.x + threadIdx.x);
     if (k > M / 2) return;  // (a thread that has ended counts as having triggered and waited)
     const C w = k > 0 ? rw[k] : cx<C>((F)0, (F)0);  // the pair's twiddles, for every transform
-    pdl_trigger();
     pdl_wait();
+    if (early) pdl_trigger();
     for (long long tr = blockIdx.y; tr < batch; tr += gridDim.y) {
         const C* zt = z + tr * z_stride;
         constexpr int OL2 = (OP == kR2CSqrMag) ? (int)kAoS : LAYOUT;
@@ -772,13 +781,13 @@ __global__ void rfft_split_kernel(const Cx<F>* z, void* out0, void* out1, const 
 template <typename F, int LAYOUT>
 __global__ void rfft_pre_kernel(const void* in0, const void* in1, Cx<F>* z, const Cx<F>* rw, int M, long long batch,
                                 long long in_stride, long long z_stride, const void* const* gin0,
-                                const void* const* gin1) {
+                                const void* const* gin1, int early) {
     using C = Cx<F>;
     const int k = (int)(blockIdx.x * blockDim.x + threadIdx.x);
     if (k > M / 2) return;  // (a thread that has ended counts as having triggered and waited)
     const C w = k > 0 ? rw[k] : cx<C>((F)0, (F)0);  // the pair's twiddles, for every transform
-    pdl_trigger();
     pdl_wait();
+    if (early) pdl_trigger();
     for (long long tr = blockIdx.y; tr < batch; tr += gridDim.y) {
         const CxIn<F, LAYOUT> in(gin0 ? gin0[tr] : in0, gin0 ? (gin1 ? gin1[tr] : nullptr) : in1,
                                  gin0 ? 0 : tr * in_stride);

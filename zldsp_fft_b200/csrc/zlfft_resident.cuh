@@ -30,10 +30,16 @@ int resident_ctas(ResidentSlots& slots, Setup&& setup) {
     return b;
 }
 
-// The common set-up: the shared-memory limit, then the occupancy query.
+// Shared memory of an SM, what each resident CTA takes of it besides its own,
+// and the most that one CTA may ask for.
+constexpr size_t kSmemPerSm = 228 * 1024, kSmemReserve = 1024, kSmemPerCta = kSmemPerSm - kSmemReserve;
+
+// The common set-up: the shared-memory limit (of `limit` bytes, where a launch
+// may ask for more than `smem`), then the occupancy query.
 template <typename K>
-int occupancy_setup(K kern, int threads, size_t smem) {
-    if (smem > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+int occupancy_setup(K kern, int threads, size_t smem, size_t limit = 0) {
+    if (limit < smem) limit = smem;
+    if (limit > 48 * 1024) cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
     int b = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kern, threads, smem) != cudaSuccess || b < 1) b = 1;
     return b;

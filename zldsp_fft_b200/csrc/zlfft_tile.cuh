@@ -1073,6 +1073,12 @@ struct TileWorker {
 };
 
 // ---------------------------------------------------------------- the kernel
+// Grids of up to half the SMs let the next kernel in before they wait: chains
+// of such calls lie side by side on idle SMs whatever their number (RFFT<float> of
+// order 7 backward, 16 tiles: 2.7 us a call against 3.0; 100 tiles, though, 3.1
+// against 3.0).
+constexpr unsigned kEarlyGrid = 74;
+
 template <typename C>
 __device__ __forceinline__ void copy_table(C* dst, const C* src, int n) {
     for (int i = (int)threadIdx.x; i < n; i += (int)blockDim.x) dst[i] = src[i];
@@ -1130,8 +1136,9 @@ __global__ void __launch_bounds__(TileCfg<F, P, OP, 128, 0, NQ>::THREADS, TileCf
             }
         }
     }
-    pdl_trigger();  // the next kernel may set up in the slots this one's CTAs leave
-    pdl_wait();     // the caller's buffers may be the kernel before us's until here
+    if (gridDim.x <= kEarlyGrid) pdl_trigger();
+    pdl_wait();  // the caller's buffers may be the kernel before us's until here
+    if (gridDim.x > kEarlyGrid) pdl_trigger();  // the next kernel may set up in the slots this one's CTAs leave
     if constexpr (Tabs::kWin) copy_table(t_win, static_cast<const C*>(a.win), N);
     __syncthreads();  // barrier initialised, table copies complete
     if constexpr (Cfg::kTMA || Cfg::kTMA1) {
