@@ -102,35 +102,67 @@ struct TileTable {
     TileLaunchFn fast[kTileTableP + 1][5][2];
 };
 
-// Transforms per thread. Two share their twiddle, window and split-twiddle
-// loads, their index arithmetic and their barriers (half of each per
-// transform), and give the scheduler two independent chains; they cost
-// registers (4 CTAs of 128 threads per SM instead of 5, with twice the
-// transforms in flight) and the separate staging buffer. Measured, complex
-// orders 9-11 (us, one -> two): STFT squared magnitudes 195.9 -> 182.1, 203.2 ->
-// 186.1, 208.2 -> 183.6; batched squared magnitudes 98.5 -> 92.5, 102.0 -> 97.2,
-// 102.4 -> 97.6; forward bins 96.7 -> 97.9 (split re/im 102.0 -> 110.2), 102.2 ->
-// 104.4, 108.3 -> 108.7 (bound by their stores); CFFTs 175.5 -> 191.7, 185.6 -> 194.8; and
-// from order 12 on the CTAs grow too large (squared magnitudes 106.0 -> 112.5).
-template <typename F, int P, int OP, bool WIN, bool FAST>
+// Transforms per thread, in a batch that fills the GPU (pair_pays). Two share their
+// twiddle, window and split-twiddle loads, their index arithmetic and their
+// barriers (half of each per transform), and give the scheduler two
+// independent chains; they cost registers (4 CTAs of 128 threads per SM
+// instead of 5, with twice the transforms in flight) and the separate staging
+// buffer. Measured, complex orders 9-11 (us, one -> two): STFT squared
+// magnitudes 195.9 -> 182.1, 203.2 -> 186.1, 208.2 -> 183.6; batched squared magnitudes
+// 98.5 -> 92.5, 102.0 -> 97.2, 102.4 -> 97.6; forward bins 96.7 -> 97.9 (split re/im
+// 102.0 -> 110.2), 102.2 -> 104.4, 108.3 -> 108.7 (bound by their stores); CFFTs 175.5 ->
+// 191.7, 185.6 -> 194.8; and from order 12 on the CTAs grow too large (squared
+// magnitudes 106.0 -> 112.5).
+template <typename F, int P, int OP, bool WIN>
 constexpr int tile_nq() {
     return sizeof(F) == 4 && P >= 9 && P <= 11 && (WIN || OP == kR2CSqrMag) ? 2 : 1;
 }
 
-template <typename F, int P, int OP, int IL, int OL, bool WIN = false, bool FAST = false>
-cudaError_t launch_tile(const TileArgs& a, cudaStream_t stream, const LaunchCtx& ctx) {
-    constexpr int NQ = tile_nq<F, P, OP, WIN, FAST>();
+// Whether a batch of `tiles` tiles (one transform per thread) runs faster with
+// two transforms per thread; cap1 and cap2 are the tiles that fill the GPU
+// with one and with two. A wave of the latter takes about 1.5 of the former, so
+// the waves decide. Measured, RFFT<float> 10 squared magnitudes (us, one / two; 740
+// and 592 tiles a wave): 1 tile 2.6 / 3.6, 296 3.7 / 4.3, 740 6.0 / 7.6; 1184 10.1 / 8.1;
+// 1480 10.2 / 12.9; 2220 14.2 / 14.7; 2368 15.7 / 14.6; 3552 22.2 / 20.8; 17760 100.5 /
+// 96.7. By itself after a pause, 74 tiles: 5.3 / 6.8.
+inline bool pair_pays(long long tiles, long long cap1, long long cap2) {
+    const long long waves1 = (tiles + cap1 - 1) / cap1;
+    const long long waves2 = ((tiles + 1) / 2 + cap2 - 1) / cap2;
+    return waves2 > 4 || 2 * waves1 > 3 * waves2;
+}
+
+// A tile kernel with NQ transforms per thread: its launch, and the CTAs of it that fit on an SM.
+template <typename F, int P, int OP, int IL, int OL, bool WIN, bool FAST, int NQ>
+struct TileLaunch {
     using Cfg = TileCfg<F, P, OP, 128, 0, NQ>;
     using Tabs = TileTabs<F, P, OP, WIN, FAST, Cfg>;
-    auto kern = tile_kernel<F, P, OP, IL, OL, false, WIN, FAST, NQ>;
-    static ResidentSlots slots;
-    const int blocks_per_sm = resident_ctas(slots, [kern] { return occupancy_setup(kern, Cfg::THREADS, Tabs::SMEM, kSmemPerCta); });
-    if (a.batch <= 0) return cudaSuccess;
-    const long long tiles = (a.batch + Cfg::TPT - 1) / Cfg::TPT;
-    const long long cap = (long long)ctx.num_sms * blocks_per_sm;
-    const unsigned grid = (unsigned)(tiles < cap ? tiles : cap);
-    if (ctx.launches) ++*ctx.launches;
-    return launch_dependent(kern, grid, Cfg::THREADS, balanced_smem(ctx, grid, blocks_per_sm, Tabs::SMEM), stream, a);
+    static int per_sm() {
+        auto kern = tile_kernel<F, P, OP, IL, OL, false, WIN, FAST, NQ>;
+        static ResidentSlots slots;
+        return resident_ctas(slots, [kern] { return occupancy_setup(kern, Cfg::THREADS, Tabs::SMEM, kSmemPerCta); });
+    }
+    static cudaError_t run(const TileArgs& a, cudaStream_t stream, const LaunchCtx& ctx) {
+        const int blocks_per_sm = per_sm();
+        if (a.batch <= 0) return cudaSuccess;
+        const long long tiles = (a.batch + Cfg::TPT - 1) / Cfg::TPT;
+        const long long cap = (long long)ctx.num_sms * blocks_per_sm;
+        const unsigned grid = (unsigned)(tiles < cap ? tiles : cap);
+        if (ctx.launches) ++*ctx.launches;
+        return launch_dependent(tile_kernel<F, P, OP, IL, OL, false, WIN, FAST, NQ>, grid, Cfg::THREADS,
+                                balanced_smem(ctx, grid, blocks_per_sm, Tabs::SMEM), stream, a);
+    }
+};
+
+template <typename F, int P, int OP, int IL, int OL, bool WIN = false, bool FAST = false>
+cudaError_t launch_tile(const TileArgs& a, cudaStream_t stream, const LaunchCtx& ctx) {
+    using One = TileLaunch<F, P, OP, IL, OL, WIN, FAST, 1>;
+    if constexpr (tile_nq<F, P, OP, WIN>() == 2) {
+        using Two = TileLaunch<F, P, OP, IL, OL, WIN, FAST, 2>;
+        const long long tiles = (a.batch + One::Cfg::TPT - 1) / One::Cfg::TPT;
+        if (pair_pays(tiles, (long long)ctx.num_sms * One::per_sm(), (long long)ctx.num_sms * Two::per_sm()))
+            return Two::run(a, stream, ctx);
+    }
+    return One::run(a, stream, ctx);
 }
 
 // ------------------------------------------------------------------ gathered tile launches
