@@ -1,8 +1,9 @@
 // Host rules of the launch headers, checked against their definitions. Host
 // code only: nvcc compiles it for sm_100a, but nothing runs on a GPU.
+#include <chrono>
 #include <cstdio>
 
-#include "zlfft_launch.cuh"
+#include "zlfft_istft.cuh"
 
 using namespace zlfft;
 
@@ -12,6 +13,19 @@ static void expect(bool ok, const char* what) {
         ++bad;
         printf("FAILED: %s\n", what);
     }
+}
+
+// The run length by trying every one: the cheapest between the shortest that
+// takes one wave of groups and 4 (K - 1), the shortest of equals.
+static long long run_by_trying(long long blocks, int k, long long sms, int groups) {
+    const long long cap = sms * groups, rmin = (blocks + cap - 1) / cap;
+    long long run = rmin, best = -1;
+    for (long long r = rmin; r <= 4LL * (k - 1); ++r) {
+        const long long g = ((blocks + r - 1) / r + sms - 1) / sms;
+        const long long cost = (r + k - 1) * (2 * g > 3 ? 2 * g : 3);
+        if (best < 0 || cost < best) best = cost, run = r;
+    }
+    return run;
 }
 
 int main() {
@@ -25,5 +39,18 @@ int main() {
         for (long long t = 8 * cap2 + 1; t <= 40 * cap2; t += 7) expect(pair_pays(t, cap1, cap2), "many waves: pairs");
     }
     printf("pairs: %s\n", bad ? "bad" : "ok");
+    // inverse STFT: the weighed runs give what trying every length gives
+    for (int k : {1, 2, 3, 4, 8, 16, 64, 512, 8192})
+        for (int groups : {1, 2, 5, 10, 15, 32})
+            for (long long sms : {148LL, 64LL})
+                for (long long blocks = 1; blocks < 4000000; blocks = blocks * 5 / 3 + 1)
+                    expect(istft_run(blocks, k, sms, groups) == run_by_trying(blocks, k, sms, groups), "run length");
+    // and take no longer for many overlapping frames than for few
+    long long sum = 0;
+    const auto t0 = std::chrono::steady_clock::now();
+    for (int i = 0; i < 20000; ++i) sum += istft_run(9000 + i, 8192, 148, 15);
+    const double us = std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t0).count() / 20000;
+    expect(us < 10 && sum > 0, "host time of the run length");
+    printf("runs: %s\n", bad ? "bad" : "ok");
     return bad ? 1 : 0;
 }

@@ -167,15 +167,36 @@ __global__ void __launch_bounds__(IstftCfg<F, P>::THREADS, 1) istft_kernel(const
         for (long long i = lt; i < hp; i += T) sig[m * hp + i] = ring[(uint32_t)((m * hp + i) & (N - 1))];
 }
 
-using IstftLaunchFn = cudaError_t (*)(const TileArgs&, const IstftArgs&, cudaStream_t, const LaunchCtx&);
-
-// One group per run of blocks. A full load takes one wave of the resident
+// Blocks per run for `blocks` blocks of K overlapping frames over num_sms SMs
+// that hold `groups` groups each. A full load takes one wave of the resident
 // groups, at least 4 (K - 1) blocks each, so that the K - 1 frames a group
 // transforms ahead of its run add at most a quarter to the work. A smaller
-// one weighs those frames against idle SMs: a run of `run` blocks costs
-// run + K - 1 frames, and a frame takes about 3 units of time on an SM whose
-// other groups idle, 2 g with g groups at work. Run r is group r / grid of CTA
-// r % grid, so that few runs still spread over all SMs.
+// one weighs those frames against idle SMs: a run of r blocks costs r + K - 1
+// frames, and a frame takes about 3 units of time on an SM whose other groups
+// idle, 2 g with g groups at work (frames of order 12: 3.5 us alone, 9.8 with five
+// groups at work, 9.8 / 3.5 = 2.8 against 10 / 3). For each g only the shortest run that needs
+// no more than g groups per SM can be the cheapest, so `groups` runs are
+// weighed, whatever K.
+inline long long istft_run(long long blocks, int k, long long num_sms, int groups) {
+    const long long longest = 4LL * (k - 1);
+    long long run = (blocks + num_sms * groups - 1) / (num_sms * groups), best = -1;
+    for (int g = groups; g >= 1; --g) {
+        const long long r = (blocks + num_sms * g - 1) / (num_sms * g);
+        if (r > longest) break;
+        const long long used = ((blocks + r - 1) / r + num_sms - 1) / num_sms;
+        const long long cost = (r + k - 1) * (2 * used > 3 ? 2 * used : 3);
+        if (best < 0 || cost < best) {
+            best = cost;
+            run = r;
+        }
+    }
+    return run;
+}
+
+using IstftLaunchFn = cudaError_t (*)(const TileArgs&, const IstftArgs&, cudaStream_t, const LaunchCtx&);
+
+// One group per run of blocks. Run r is group r / grid of CTA r % grid, so that
+// few runs still spread over all SMs.
 template <typename F, int P, int IL>
 cudaError_t launch_istft(const TileArgs& a, const IstftArgs& o, cudaStream_t stream, const LaunchCtx& ctx) {
     using Cfg = IstftCfg<F, P>;
@@ -184,19 +205,8 @@ cudaError_t launch_istft(const TileArgs& a, const IstftArgs& o, cudaStream_t str
     (void)resident_ctas(slots, [kern] { return occupancy_setup(kern, Cfg::THREADS, Cfg::SMEM); });
     if (o.n_frames <= 0 || o.blocks <= 0) return cudaSuccess;
     IstftArgs oo = o;
-    const long long cap = (long long)ctx.num_sms * Cfg::GROUPS;
-    const long long rmin = (o.blocks + cap - 1) / cap;
-    long long run = rmin, best = -1;
-    for (long long r = rmin; r <= 4LL * (o.k - 1); ++r) {
-        const long long g = ((o.blocks + r - 1) / r + ctx.num_sms - 1) / ctx.num_sms;
-        const long long cost = (r + o.k - 1) * (2 * g > 3 ? 2 * g : 3);
-        if (best < 0 || cost < best) {
-            best = cost;
-            run = r;
-        }
-    }
-    oo.run = run;
-    const long long groups = (o.blocks + run - 1) / run;
+    oo.run = istft_run(o.blocks, o.k, ctx.num_sms, Cfg::GROUPS);
+    const long long groups = (o.blocks + oo.run - 1) / oo.run;
     const long long grid = groups < ctx.num_sms ? groups : ctx.num_sms;
     if (ctx.launches) ++*ctx.launches;
     return launch_dependent(kern, (unsigned)grid, Cfg::THREADS, Cfg::SMEM, stream, a, oo);
