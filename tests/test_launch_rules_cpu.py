@@ -21,4 +21,5 @@ def test_launch_rules(tmp_path):
     r = subprocess.run(cmd, capture_output=True, text=True, timeout=600)
     assert r.returncode == 0, r.stderr[-3000:]
     r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
-    assert r.returncode == 0 and "pairs: ok" in r.stdout and "runs: ok" in r.stdout, r.stdout[-2000:] + r.stderr
+    assert r.returncode == 0, r.stdout[-2000:] + r.stderr
+    assert all(f"{rule}: ok" in r.stdout for rule in ("pairs", "runs", "single")), r.stdout

@@ -71,7 +71,11 @@ struct OlaSink {
 // 1420 us for 131069 frames of order 12 at hop N / 4 against 1365, 319 against
 // 289 for 4096 frames of order 14. A copy per CTA would not fit.) The bins are
 // read directly: staging them costs a group.
-template <typename F, int P>
+//
+// Where every group transforms one frame and few of them share an SM, copying
+// the tables costs more than it saves, and a CTA is one group that reads them
+// from global memory (SHARED false; istft_single).
+template <typename F, int P, bool SHARED>
 struct IstftCfg {
     using C = Cx<F>;
     static constexpr int N = 1 << P;                  // complex points (frame length / 2)
@@ -87,28 +91,30 @@ struct IstftCfg {
     static constexpr int by_regs = 65536 / (REGS * (T > 0 ? T : 1)), by_smem = (int)(kSm / GBYTES);
     static constexpr int G0 = by_regs < by_smem ? by_regs : by_smem;
     static constexpr int G1 = G0 > 1024 / (T > 0 ? T : 1) ? 1024 / (T > 0 ? T : 1) : G0;
-    static constexpr int GROUPS = T > 32 && G1 > 15 ? 15 : (G1 > 0 ? G1 : 1);
+    static constexpr int GROUPS = !SHARED ? 1 : T > 32 && G1 > 15 ? 15 : (G1 > 0 ? G1 : 1);
     static constexpr int THREADS = T * GROUPS;
     static constexpr size_t BASE = GBYTES * GROUPS;
     static constexpr size_t cxs = sizeof(C);
     static constexpr size_t mid_b = Tile::TW_MID * cxs, rw_b = ((N / 2 + 1) * cxs + 15) / 16 * 16,
                             h_b = ((N + 1) * cxs + 15) / 16 * 16, w_b = N * cxs;
-    static constexpr bool kMid = BASE + mid_b <= kSm;
+    static constexpr bool kMid = SHARED && BASE + mid_b <= kSm;
     static constexpr size_t O_MID = BASE, O_RW = O_MID + (kMid ? mid_b : 0);
-    static constexpr bool kRw = O_RW + rw_b <= kSm;
+    static constexpr bool kRw = SHARED && O_RW + rw_b <= kSm;
     static constexpr size_t O_H = O_RW + (kRw ? rw_b : 0);
-    static constexpr bool kH = O_H + h_b <= kSm;
+    static constexpr bool kH = SHARED && O_H + h_b <= kSm;
     static constexpr size_t O_W = O_H + (kH ? h_b : 0);
-    static constexpr bool kW = O_W + w_b <= kSm;
+    static constexpr bool kW = SHARED && O_W + w_b <= kSm;
     static constexpr size_t SMEM = O_W + (kW ? w_b : 0);
     static constexpr int TABS = (kMid ? kTabMid : 0) | (kRw ? kTabRw : 0);
+    static constexpr int MINB = SHARED ? 1 : Tile::MINB;
 };
 
-template <typename F, int P, int IL>
-__global__ void __launch_bounds__(IstftCfg<F, P>::THREADS, 1) istft_kernel(const TileArgs a, const IstftArgs o) {
-    using Cfg = IstftCfg<F, P>;
+template <typename F, int P, int IL, bool SHARED>
+__global__ void __launch_bounds__(IstftCfg<F, P, SHARED>::THREADS, IstftCfg<F, P, SHARED>::MINB)
+    istft_kernel(const TileArgs a, const IstftArgs o) {
+    using Cfg = IstftCfg<F, P, SHARED>;
     using C = Cx<F>;
-    using W = TileWorker<F, P, kC2RBwd, IL, kAoS, Cfg::T, false, false, false, false, 0, 1, Cfg::TABS, true>;
+    using W = TileWorker<F, P, kC2RBwd, IL, kAoS, Cfg::T, false, false, false, false, 0, 1, Cfg::TABS, SHARED>;
     constexpr int N = Cfg::N, T = Cfg::T;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int grp = (int)threadIdx.x / T, lt = (int)threadIdx.x % T;
@@ -133,9 +139,11 @@ __global__ void __launch_bounds__(IstftCfg<F, P>::THREADS, 1) istft_kernel(const
     // The bins come from HBM with nothing else to do meanwhile: one thread asks
     // L2 for the next frame's before this one is transformed (1639 -> 1365 us for
     // 131069 frames of order 12 at hop N / 4; with it the shared tables are worth
-    // 4% there, without it nothing).
+    // 4% there, without it nothing). A CTA of one group and one frame only asks
+    // where it is a single warp (order 10, 74 frames 6.3 us against 7.9; order 13
+    // 7.4 against 6.1).
     auto prefetch = [&](long long f) {
-        if (lt != 0 || f > f1 || m0 >= m1) return;
+        if ((!SHARED && T > 32) || lt != 0 || f > f1 || m0 >= m1) return;
         if constexpr (IL == kSoA) {
             prefetch_l2(static_cast<const F*>(a.in0) + f * a.in_stride, (N + 1) * sizeof(F));
             prefetch_l2(static_cast<const F*>(a.in1) + f * a.in_stride, (N + 1) * sizeof(F));
@@ -193,23 +201,46 @@ inline long long istft_run(long long blocks, int k, long long num_sms, int group
     return run;
 }
 
+// Whether `runs` runs of `frames` frames each go to CTAs of one group: one frame
+// each, up to two thirds of the groups that fit, and more than one of those per SM
+// (else the two kernels hardly differ). Measured at hop N, orders 10 / 11 / 12 / 13,
+// groups that share tables against one group a CTA, us: one frame by itself 8.9 / 8.3 /
+// 9.7 / 10.2 against 6.7 / 6.0 / 8.0 / 8.1, in a chain of calls 5.4 / 5.1 / 6.7 / 7.1
+// against 4.9 / 4.1 / 6.2 / 6.1; 148 frames in a chain 7.5 / 6.7 / 8.2 / 8.9 against 6.4 /
+// 4.6 / 6.9 / 8.6. Of several frames a group, the tables and the prefetch pay: order
+// 12, hop N / 4, 16 frames 17.8 against 20.8.
+inline bool istft_single(long long runs, long long frames, long long num_sms, int groups) {
+    return groups > 1 && frames == 1 && 3 * runs <= 2 * num_sms * groups;
+}
+
 using IstftLaunchFn = cudaError_t (*)(const TileArgs&, const IstftArgs&, cudaStream_t, const LaunchCtx&);
+
+template <typename F, int P, int IL, bool SHARED>
+cudaError_t launch_istft_kernel(const TileArgs& a, const IstftArgs& o, long long grid, cudaStream_t stream,
+                                const LaunchCtx& ctx) {
+    using Cfg = IstftCfg<F, P, SHARED>;
+    auto kern = istft_kernel<F, P, IL, SHARED>;
+    static ResidentSlots slots;
+    const int per_sm =
+        resident_ctas(slots, [kern] { return occupancy_setup(kern, Cfg::THREADS, Cfg::SMEM, kSmemPerCta); });
+    if (ctx.launches) ++*ctx.launches;
+    return launch_dependent(kern, (unsigned)grid, Cfg::THREADS, balanced_smem(ctx, grid, per_sm, Cfg::SMEM), stream, a,
+                            o);
+}
 
 // One group per run of blocks. Run r is group r / grid of CTA r % grid, so that
 // few runs still spread over all SMs.
 template <typename F, int P, int IL>
 cudaError_t launch_istft(const TileArgs& a, const IstftArgs& o, cudaStream_t stream, const LaunchCtx& ctx) {
-    using Cfg = IstftCfg<F, P>;
-    auto kern = istft_kernel<F, P, IL>;
-    static ResidentSlots slots;
-    (void)resident_ctas(slots, [kern] { return occupancy_setup(kern, Cfg::THREADS, Cfg::SMEM); });
     if (o.n_frames <= 0 || o.blocks <= 0) return cudaSuccess;
+    constexpr int GROUPS = IstftCfg<F, P, true>::GROUPS;
     IstftArgs oo = o;
-    oo.run = istft_run(o.blocks, o.k, ctx.num_sms, Cfg::GROUPS);
-    const long long groups = (o.blocks + oo.run - 1) / oo.run;
-    const long long grid = groups < ctx.num_sms ? groups : ctx.num_sms;
-    if (ctx.launches) ++*ctx.launches;
-    return launch_dependent(kern, (unsigned)grid, Cfg::THREADS, Cfg::SMEM, stream, a, oo);
+    oo.run = istft_run(o.blocks, o.k, ctx.num_sms, GROUPS);
+    const long long runs = (o.blocks + oo.run - 1) / oo.run;
+    const long long ahead = oo.run + o.k - 1;  // frames that a whole run takes
+    if (istft_single(runs, ahead < o.n_frames ? ahead : o.n_frames, ctx.num_sms, GROUPS))
+        return launch_istft_kernel<F, P, IL, false>(a, oo, runs, stream, ctx);
+    return launch_istft_kernel<F, P, IL, true>(a, oo, runs < ctx.num_sms ? runs : ctx.num_sms, stream, ctx);
 }
 
 // [complex order][input layout]; null where the order has no ISTFT kernel
@@ -221,7 +252,7 @@ template <typename F, int... Ps>
 void fill_istft_orders(IstftTable& t, std::integer_sequence<int, Ps...>) {
     (
         [&] {
-            if constexpr (IstftCfg<F, Ps>::kOK) {
+            if constexpr (IstftCfg<F, Ps, true>::kOK) {
                 t.fn[Ps][kAoS] = launch_istft<F, Ps, kAoS>;
                 t.fn[Ps][kSoA] = launch_istft<F, Ps, kSoA>;
             }
