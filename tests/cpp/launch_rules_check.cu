@@ -39,6 +39,35 @@ int main() {
         for (long long t = 8 * cap2 + 1; t <= 40 * cap2; t += 7) expect(pair_pays(t, cap1, cap2), "many waves: pairs");
     }
     printf("pairs: %s\n", bad ? "bad" : "ok");
+    // launches that begin when the one before is done: short tiles in the second
+    // of two waves, passes of one to four waves whose last is under half full;
+    // none beside other launches of the call
+    const LaunchCtx alone{148, nullptr, false}, beside{148, nullptr, true};
+    for (long long cap : {148LL, 444LL, 740LL}) {
+        for (long long n = 1; n <= 6 * cap; ++n) {
+            expect(tile_overlaps(alone, 8, n, cap) == !(n > cap && n < 2 * cap), "short tiles");
+            expect(tile_overlaps(alone, 9, n, cap) && tile_overlaps(beside, 8, n, cap), "other tiles");
+            const bool ragged = n > cap && n < 4 * cap && n % cap != 0 && n % cap < (cap + 1) / 2;
+            expect(pass_overlaps(alone, n, cap) == !ragged, "passes");
+            expect(pass_overlaps(beside, n, cap), "passes of two chunks");
+        }
+    }
+    // shared memory asked for: the even share of CTAs fits an SM and one more
+    // does not, where more would fit, but two even shares would not
+    for (int per_sm = 1; per_sm <= 24; ++per_sm) {
+        const size_t own = kSmemPerSm / per_sm / 1024 * 1024 - kSmemReserve;
+        for (long long grid = 1; grid <= 148LL * per_sm; ++grid) {
+            const int k = (int)((grid + 147) / 148);
+            const size_t got = balanced_smem(alone, grid, per_sm, own);
+            const size_t each = got + kSmemReserve;
+            if (k < per_sm && 2 * k > per_sm)
+                expect(each % 1024 == 0 && k * each <= kSmemPerSm && (2 * k) * each > kSmemPerSm && got <= kSmemPerCta, "share");
+            else
+                expect(got == own, "own size");
+            expect(balanced_smem(beside, grid, per_sm, own) == own, "own size beside others");
+        }
+    }
+    printf("launches: %s\n", bad ? "bad" : "ok");
     // inverse STFT: the weighed runs give what trying every length gives
     for (int k : {1, 2, 3, 4, 8, 16, 64, 512, 8192})
         for (int groups : {1, 2, 5, 10, 15, 32})

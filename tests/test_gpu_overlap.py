@@ -59,7 +59,9 @@ def test_chained_call_is_not_slower_than_alone(kind, order, dtype, batch):
 # grids of three CTAs per SM where more would fit, of a few ragged waves, of single items
 @pytest.mark.parametrize("kind,order,batch", [
     (Z.C2C, 6, 444 * 32 - 5), (Z.C2C, 9, 370 * 4 - 1), (Z.C2C, 11, 440), (Z.R2C, 12, 400), (Z.R2C, 7, 443 * 32 + 3),
-    (Z.C2C, 16, 16), (Z.C2C, 16, 40), (Z.C2C, 19, 5), (Z.C2C, 21, 1), (Z.R2C, 19, 2), (Z.R2C, 17, 9)])
+    (Z.C2C, 16, 16), (Z.C2C, 16, 40), (Z.C2C, 19, 5), (Z.C2C, 21, 1), (Z.R2C, 19, 2), (Z.R2C, 17, 9),
+    (Z.C2C, 8, 1184 * 8 - 1), (Z.R2C, 7, 888 * 32 + 1),  # short tiles, a second wave not full
+    (Z.C2C, 16, 300), (Z.R2C, 18, 200)])                 # more than two chunks on two streams
 def test_bits_of_chained_calls(oracle, kind, order, batch):
     """Each call reads what the one before wrote, with nothing between them;
     the inputs change from round to round, so a call that reads too early finds

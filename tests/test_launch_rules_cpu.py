@@ -22,4 +22,4 @@ def test_launch_rules(tmp_path):
     assert r.returncode == 0, r.stderr[-3000:]
     r = subprocess.run([exe], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout[-2000:] + r.stderr
-    assert all(f"{rule}: ok" in r.stdout for rule in ("pairs", "runs", "single")), r.stdout
+    assert all(f"{rule}: ok" in r.stdout for rule in ("pairs", "launches", "runs", "single")), r.stdout
