@@ -81,15 +81,15 @@ int main() {
     const double us = std::chrono::duration<double, std::micro>(std::chrono::steady_clock::now() - t0).count() / 20000;
     expect(us < 10 && sum > 0, "host time of the run length");
     printf("runs: %s\n", bad ? "bad" : "ok");
-    // CTAs of one group: for single frames on SMs that hold several groups, few of them
-    for (int groups : {2, 3, 5, 10, 21}) {
-        const long long line = 2LL * 148 * groups / 3;
-        for (long long runs : {1LL, 2LL, line - 1, line}) {
-            expect(istft_single(runs, 1, 148, groups), "few single frames");
-            expect(!istft_single(runs, 2, 148, groups), "several frames a group");
-            expect(!istft_single(runs, 1, 148, 1), "one group on an SM");
+    // CTAs of one group: one wave of single frames, on SMs that hold several groups
+    for (int groups : {4, 5, 7, 10, 21}) {
+        const long long slots = 148LL * (groups - 1);
+        for (long long runs : {1LL, 2LL, slots - 1, slots}) {
+            expect(istft_single(runs, 1, slots, groups), "a wave of single frames");
+            expect(!istft_single(runs, 2, slots, groups), "several frames a group");
+            for (int few = 1; few <= 3; ++few) expect(!istft_single(runs, 1, slots, few), "few groups on an SM");
         }
-        expect(!istft_single(line + 1, 1, 148, groups), "many single frames");
+        expect(!istft_single(slots + 1, 1, slots, groups), "more than a wave");
     }
     printf("single: %s\n", bad ? "bad" : "ok");
     return bad ? 1 : 0;

@@ -1,7 +1,6 @@
 """Inverse STFT of few frames without overlap: CTAs of one group each. The
-sequential loop's bits on both sides of the rule (two thirds of the groups that
-fit on the SMs, one frame each), with and without filter and window, AoS and
-split bins."""
+sequential loop's bits on both sides of the rule (one wave of groups, one frame
+each), with and without filter and window, AoS and split bins."""
 import numpy as np
 import pytest
 
@@ -33,13 +32,13 @@ def test_bits_on_both_sides(oracle, order, prec, extras, layout):
     n = 1 << order
     nb = n // 2 + 1
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    line = 2 * sms * GROUPS[order, prec] // 3
+    full = sms * GROUPS[order, prec]
     rng = np.random.default_rng(9400 + order)
     plan = Z.Plan(Z.R2C, order, dt)
     filt = (rng.uniform(-1, 1, nb) + 1j * rng.uniform(-1, 1, nb)).astype(cdt) if extras else None
     win = rng.uniform(0, 1, n).astype(dt) if extras else None
     fd, wd = (None if a is None else G.dev(a.view(dt)) for a in (filt, win))
-    for count in sorted({1, 3, line, line + 1}):
+    for count in sorted({1, 3, full // 2 + 1, full, full + 1}):
         bins = (rng.uniform(-1, 1, (count, nb)) + 1j * rng.uniform(-1, 1, (count, nb))).astype(cdt)
         if layout == Z.AOS:
             a, b = G.dev(bins.view(dt)), None

@@ -201,32 +201,36 @@ inline long long istft_run(long long blocks, int k, long long num_sms, int group
     return run;
 }
 
-// Whether `runs` runs of `frames` frames each go to CTAs of one group: one frame
-// each, up to two thirds of the groups that fit, and more than one of those per SM
-// (else the two kernels hardly differ). Measured at hop N, orders 10 / 11 / 12 / 13,
-// groups that share tables against one group a CTA, us: one frame by itself 8.9 / 8.3 /
-// 9.7 / 10.2 against 6.7 / 6.0 / 8.0 / 8.1, in a chain of calls 5.4 / 5.1 / 6.7 / 7.1
-// against 4.9 / 4.1 / 6.2 / 6.1; 148 frames in a chain 7.5 / 6.7 / 8.2 / 8.9 against 6.4 /
-// 4.6 / 6.9 / 8.6. Of several frames a group, the tables and the prefetch pay: order
-// 12, hop N / 4, 16 frames 17.8 against 20.8.
-inline bool istft_single(long long runs, long long frames, long long num_sms, int groups) {
-    return groups > 1 && frames == 1 && 3 * runs <= 2 * num_sms * groups;
+// Whether `runs` runs of `frames` frames each go to CTAs of one group, `slots` of
+// which fill the GPU: one frame each, one wave, where an SM holds several (`groups`
+// that share tables). Measured at hop N, orders 10 / 11 / 12, groups that share
+// tables against one group a CTA, us: one frame by itself 9.2 / 8.3 / 10.1 against 7.1 / 6.0 /
+// 8.4, in a chain of calls 5.5 / 5.1 / 6.7 against 5.1 / 4.1 / 6.4; 148 frames in a chain 7.6 /
+// 6.7 / 8.2 against 6.3 / 4.6 / 6.9, 740 frames 8.2 / 8.6 / 12.2 against 6.8 / 7.0 / 11.4. Order
+// 13 (two groups) gains up to 4 frames and loses 7-14% at 8-100. Of several frames a
+// group, the tables and the prefetch pay: order 12, hop N / 4, 16 frames 17.8
+// against 20.8.
+inline bool istft_single(long long runs, long long frames, long long slots, int groups) {
+    return groups > 3 && frames == 1 && runs <= slots;
 }
 
 using IstftLaunchFn = cudaError_t (*)(const TileArgs&, const IstftArgs&, cudaStream_t, const LaunchCtx&);
 
+// The kernel's launch, and the CTAs of it that fit on an SM.
 template <typename F, int P, int IL, bool SHARED>
-cudaError_t launch_istft_kernel(const TileArgs& a, const IstftArgs& o, long long grid, cudaStream_t stream,
-                                const LaunchCtx& ctx) {
+struct IstftLaunch {
     using Cfg = IstftCfg<F, P, SHARED>;
-    auto kern = istft_kernel<F, P, IL, SHARED>;
-    static ResidentSlots slots;
-    const int per_sm =
-        resident_ctas(slots, [kern] { return occupancy_setup(kern, Cfg::THREADS, Cfg::SMEM, kSmemPerCta); });
-    if (ctx.launches) ++*ctx.launches;
-    return launch_dependent(kern, (unsigned)grid, Cfg::THREADS, balanced_smem(ctx, grid, per_sm, Cfg::SMEM), stream, a,
-                            o);
-}
+    static int per_sm() {
+        auto kern = istft_kernel<F, P, IL, SHARED>;
+        static ResidentSlots slots;
+        return resident_ctas(slots, [kern] { return occupancy_setup(kern, Cfg::THREADS, Cfg::SMEM, kSmemPerCta); });
+    }
+    static cudaError_t run(const TileArgs& a, const IstftArgs& o, long long grid, cudaStream_t stream, const LaunchCtx& ctx) {
+        const size_t smem = balanced_smem(ctx, grid, per_sm(), Cfg::SMEM);
+        if (ctx.launches) ++*ctx.launches;
+        return launch_dependent(istft_kernel<F, P, IL, SHARED>, (unsigned)grid, Cfg::THREADS, smem, stream, a, o);
+    }
+};
 
 // One group per run of blocks. Run r is group r / grid of CTA r % grid, so that
 // few runs still spread over all SMs.
@@ -238,9 +242,10 @@ cudaError_t launch_istft(const TileArgs& a, const IstftArgs& o, cudaStream_t str
     oo.run = istft_run(o.blocks, o.k, ctx.num_sms, GROUPS);
     const long long runs = (o.blocks + oo.run - 1) / oo.run;
     const long long ahead = oo.run + o.k - 1;  // frames that a whole run takes
-    if (istft_single(runs, ahead < o.n_frames ? ahead : o.n_frames, ctx.num_sms, GROUPS))
-        return launch_istft_kernel<F, P, IL, false>(a, oo, runs, stream, ctx);
-    return launch_istft_kernel<F, P, IL, true>(a, oo, runs < ctx.num_sms ? runs : ctx.num_sms, stream, ctx);
+    using Single = IstftLaunch<F, P, IL, false>;
+    if (istft_single(runs, ahead < o.n_frames ? ahead : o.n_frames, (long long)ctx.num_sms * Single::per_sm(), GROUPS))
+        return Single::run(a, oo, runs, stream, ctx);
+    return IstftLaunch<F, P, IL, true>::run(a, oo, runs < ctx.num_sms ? runs : ctx.num_sms, stream, ctx);
 }
 
 // [complex order][input layout]; null where the order has no ISTFT kernel
