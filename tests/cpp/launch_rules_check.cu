@@ -82,14 +82,14 @@ int main() {
     expect(us < 10 && sum > 0, "host time of the run length");
     printf("runs: %s\n", bad ? "bad" : "ok");
     // CTAs of one group: one wave of single frames, on SMs that hold several groups
-    for (int groups : {4, 5, 7, 10, 21}) {
-        const long long slots = 148LL * (groups - 1);
+    for (int groups = 1; groups <= 21; ++groups) {
+        expect(istft_has_single(groups) == (groups >= 4), "sizes with single groups");
+        const long long slots = 148LL * groups;
         for (long long runs : {1LL, 2LL, slots - 1, slots}) {
-            expect(istft_single(runs, 1, slots, groups), "a wave of single frames");
-            expect(!istft_single(runs, 2, slots, groups), "several frames a group");
-            for (int few = 1; few <= 3; ++few) expect(!istft_single(runs, 1, slots, few), "few groups on an SM");
+            expect(istft_single(runs, 1, slots), "a wave of single frames");
+            expect(!istft_single(runs, 2, slots), "several frames a group");
         }
-        expect(!istft_single(slots + 1, 1, slots, groups), "more than a wave");
+        expect(!istft_single(slots + 1, 1, slots), "more than a wave");
     }
     printf("single: %s\n", bad ? "bad" : "ok");
     return bad ? 1 : 0;

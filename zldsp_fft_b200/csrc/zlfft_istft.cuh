@@ -201,18 +201,17 @@ inline long long istft_run(long long blocks, int k, long long num_sms, int group
     return run;
 }
 
-// Whether `runs` runs of `frames` frames each go to CTAs of one group, `slots` of
-// which fill the GPU: one frame each, one wave, where an SM holds several (`groups`
-// that share tables). Measured at hop N, orders 10 / 11 / 12, groups that share
+// Sizes that have a kernel of one group per CTA (of `groups` that share tables on an SM
+// otherwise), and whether `runs` runs of `frames` frames each go to it, `slots` of its
+// CTAs filling the GPU: one frame each, one wave. Measured at hop N, orders 10 / 11 / 12, groups that share
 // tables against one group a CTA, us: one frame by itself 9.2 / 8.3 / 10.1 against 7.1 / 6.0 /
 // 8.4, in a chain of calls 5.5 / 5.1 / 6.7 against 5.1 / 4.1 / 6.4; 148 frames in a chain 7.6 /
 // 6.7 / 8.2 against 6.3 / 4.6 / 6.9, 740 frames 8.2 / 8.6 / 12.2 against 6.8 / 7.0 / 11.4. Order
 // 13 (two groups) gains up to 4 frames and loses 7-14% at 8-100. Of several frames a
 // group, the tables and the prefetch pay: order 12, hop N / 4, 16 frames 17.8
 // against 20.8.
-inline bool istft_single(long long runs, long long frames, long long slots, int groups) {
-    return groups > 3 && frames == 1 && runs <= slots;
-}
+constexpr bool istft_has_single(int groups) { return groups > 3; }
+inline bool istft_single(long long runs, long long frames, long long slots) { return frames == 1 && runs <= slots; }
 
 using IstftLaunchFn = cudaError_t (*)(const TileArgs&, const IstftArgs&, cudaStream_t, const LaunchCtx&);
 
@@ -242,9 +241,11 @@ cudaError_t launch_istft(const TileArgs& a, const IstftArgs& o, cudaStream_t str
     oo.run = istft_run(o.blocks, o.k, ctx.num_sms, GROUPS);
     const long long runs = (o.blocks + oo.run - 1) / oo.run;
     const long long ahead = oo.run + o.k - 1;  // frames that a whole run takes
-    using Single = IstftLaunch<F, P, IL, false>;
-    if (istft_single(runs, ahead < o.n_frames ? ahead : o.n_frames, (long long)ctx.num_sms * Single::per_sm(), GROUPS))
-        return Single::run(a, oo, runs, stream, ctx);
+    if constexpr (istft_has_single(GROUPS)) {
+        using Single = IstftLaunch<F, P, IL, false>;
+        if (istft_single(runs, ahead < o.n_frames ? ahead : o.n_frames, (long long)ctx.num_sms * Single::per_sm()))
+            return Single::run(a, oo, runs, stream, ctx);
+    }
     return IstftLaunch<F, P, IL, true>::run(a, oo, runs < ctx.num_sms ? runs : ctx.num_sms, stream, ctx);
 }
 
