@@ -1,13 +1,11 @@
 """Squared magnitudes and STFT frames with one or two transforms per thread, by
 the size of the batch: the oracle's bits on both sides of each line and with a
-last tile that is not full, and small batches that take no longer than forward
-bins (which load the same and store twice as much)."""
+last tile that is not full."""
 import numpy as np
 import pytest
 
 import zldsp_fft_b200 as Z
 from tests import gpu_util as G
-from tests.test_gpu_overlap import _us_per_call
 
 pytestmark = pytest.mark.gpu
 
@@ -50,20 +48,3 @@ def test_bits_on_both_sides_of_the_lines(oracle, order):
             assert np.array_equal(got[rows] if c == 1 else got.view(np.complex64)[rows], want), (batch, op)
             assert bool((got[batch] == 7.0).all())
     assert plan.device_status() == 0
-
-
-@pytest.mark.parametrize("order", [10, 11, 12])
-@pytest.mark.parametrize("tiles", [1, 74, 148, 740])
-def test_small_batches_are_not_slower_than_bins(order, tiles):
-    import torch
-    n = 1 << order
-    batch = tiles * (128 // ((n // 2) // 16))
-    plan = Z.Plan(Z.R2C, order, np.float32)
-    x = torch.rand(batch * n, device="cuda")
-    y = torch.zeros(batch * (n + 2), device="cuda")
-
-    def run(op):
-        return lambda st: plan.exec_device(op, Z.AOS, Z.AOS, x.data_ptr(), None, y.data_ptr(), None, batch, stream=st)
-    for between in (False, True):
-        sq, bins = _us_per_call(run(Z.FORWARD_SQR_MAG), between), _us_per_call(run(Z.FORWARD), between)
-        assert sq <= 1.08 * bins, (sq, bins, between)

@@ -1073,15 +1073,17 @@ struct TileWorker {
 };
 
 // ---------------------------------------------------------------- the kernel
-// Grids of up to half the SMs let the next kernel in before they wait: chains
-// of such calls lie side by side on idle SMs whatever their number (RFFT<float> of
-// order 7 backward, 16 tiles: 2.7 us a call against 3.0; 100 tiles, though, 3.1
-// against 3.0).
-constexpr unsigned kEarlyGrid = 74;
+// Small grids let the next kernel in before they wait: chains of such calls lie
+// side by side on idle SMs (RFFT<float> of order 7 backward, 16 tiles: 2.7 us a
+// call against 3.0; but 74 and 100 tiles of RFFT<float> 10 forward 2.8 against 2.7,
+// of RFFT<float> 13 squared magnitudes 3.6-4.3 against 3.3, 4.5 against 3.9).
+constexpr unsigned kEarlyGrid = 32;
 
-template <typename C>
+// Copies a table with the threads from SKIP on.
+template <int SKIP = 0, typename C>
 __device__ __forceinline__ void copy_table(C* dst, const C* src, int n) {
-    for (int i = (int)threadIdx.x; i < n; i += (int)blockDim.x) dst[i] = src[i];
+    const int first = (int)threadIdx.x >= SKIP ? (int)threadIdx.x - SKIP : n;
+    for (int i = first; i < n; i += (int)blockDim.x - SKIP) dst[i] = src[i];
 }
 
 template <typename F, int P, int OP, int IL, int OL, bool GATHER = false, bool WIN = false, bool FAST = false,
@@ -1097,8 +1099,17 @@ __global__ void __launch_bounds__(TileCfg<F, P, OP, 128, 0, NQ>::THREADS, TileCf
     C* t_mid = reinterpret_cast<C*>(smem_raw + Tabs::OFF_MID);
     C* t_rw = reinterpret_cast<C*>(smem_raw + Tabs::OFF_RW);
     C* t_win = reinterpret_cast<C*>(smem_raw + Tabs::OFF_WIN);
-    if constexpr (Tabs::kMid) copy_table(t_mid, static_cast<const C*>(a.tws), Cfg::TW_MID);
-    if constexpr (Tabs::kRw) copy_table(t_rw, static_cast<const C*>(a.rw), N / 2 + 1);
+    // The first warp issues the bulk copies. It takes no part in short table copies: waiting for
+    // those loads would put the first tile's behind them. Measured, one transform after a
+    // pause (us, all warps copy -> all but the first): CFFT<float> 9 / 11 4.5 -> 3.9, 4.5 -> 4.1,
+    // RFFT<float> 10 forward 5.4 -> 4.6, RFFT<double> 12 7.8 -> 7.2 (592 of them 16.3 -> 15.2). Long
+    // copies need every warp: RFFT<float> 12 forward, 12 entries per thread without the
+    // first warp, 5.4 -> 6.1. So do 16 warps (order 14, plain, 592 transforms 55.6 -> 58.1).
+    constexpr int kEntries = (Tabs::kMid ? Cfg::TW_MID : 0) + (Tabs::kRw ? N / 2 + 1 : 0) + (Tabs::kWin ? N : 0);
+    constexpr bool kFirstIssues = (Cfg::kTMA || Cfg::kTMA1) && P < 14 && kEntries > 0 && kEntries <= 6 * (Cfg::THREADS - 32);
+    constexpr int kSkip = kFirstIssues ? 32 : 0;
+    if constexpr (Tabs::kMid) copy_table<kSkip>(t_mid, static_cast<const C*>(a.tws), Cfg::TW_MID);
+    if constexpr (Tabs::kRw) copy_table<kSkip>(t_rw, static_cast<const C*>(a.rw), N / 2 + 1);
     W w(a, smem_raw, t_mid, t_rw, t_win);
 
     // ---- TMA staging of each tile's input (one tile ahead)
@@ -1139,9 +1150,12 @@ __global__ void __launch_bounds__(TileCfg<F, P, OP, 128, 0, NQ>::THREADS, TileCf
     if (gridDim.x <= kEarlyGrid) pdl_trigger();
     pdl_wait();  // the caller's buffers may be the kernel before us's until here
     if (gridDim.x > kEarlyGrid) pdl_trigger();  // the next kernel may set up in the slots this one's CTAs leave
-    if constexpr (Tabs::kWin) copy_table(t_win, static_cast<const C*>(a.win), N);
+    if constexpr (kFirstIssues) {
+        if (use_tma) issue(blockIdx.x);  // (by the warp of the thread that initialised the barrier)
+    }
+    if constexpr (Tabs::kWin) copy_table<kSkip>(t_win, static_cast<const C*>(a.win), N);
     __syncthreads();  // barrier initialised, table copies complete
-    if constexpr (Cfg::kTMA || Cfg::kTMA1) {
+    if constexpr ((Cfg::kTMA || Cfg::kTMA1) && !kFirstIssues) {
         if (use_tma) issue(blockIdx.x);
     }
     uint32_t phase = 0;
